@@ -42,6 +42,13 @@ cudaError_t launch_piv2d(const Piv2dArgs& a, int alg, cudaStream_t s, std::strin
 
 int device_sm_count(int device);
 
+// the warp kernels' launches per FFT length (mqp_piv2d_w*.cu, mqp_piv2d_b*.cu)
+struct Piv2dBatch;
+cudaError_t launch_piv2d_w64(const Piv2dArgs& a, int alg, bool prune, cudaStream_t s, std::string& err);
+cudaError_t launch_piv2d_w32(const Piv2dArgs& a, int alg, bool prune, cudaStream_t s, std::string& err);
+cudaError_t launch_piv2d_b64(const Piv2dBatch& b, cudaStream_t s, std::string& err);
+cudaError_t launch_piv2d_b32(const Piv2dBatch& b, cudaStream_t s, std::string& err);
+
 // One persistent launch of the fused 2D kernel over the IAs of many image
 // pairs that share a kernel variant (N, prune, alg, dtype): items[k] (device
 // array) is pair k's arguments, prefix[k] the first work-queue index of its

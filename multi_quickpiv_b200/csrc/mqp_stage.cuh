@@ -104,6 +104,10 @@ __device__ __forceinline__ bool stage_wait(uint64_t* mbar, unsigned parity) {
 #endif
 }
 
+// Host: the tensor map of img2, and whether staging is on (mqp_piv2d.cu).
+bool stage_tensor_map(CUtensorMap* m, const void* img, long long H, long long W, int N);
+bool stage_enabled();
+
 // The tile's first row for a window whose pad row 0 is image row g01.
 __host__ __device__ __forceinline__ int stage_x0(int g01) { return g01 & ~3; }
 
