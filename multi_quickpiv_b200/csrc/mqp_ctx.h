@@ -45,7 +45,7 @@ struct mqp_ctx {
   cudaStream_t stream = nullptr;
   std::string last_error;
   std::mutex mu;
-  mqp_host::DevBuf img1, img2, mask, mask_skip, II1, IIg, IIg2, VF, SN, pred, planes, status, iscratch, scratch3d;
+  mqp_host::DevBuf img1, img2, mask, mask_skip, II1, IIg, IIg2, wmap, VF, SN, pred, planes, status, iscratch, scratch3d;
   mqp_host::DevBuf passVF[2];  // vectors of the coarse passes of a multi-pass refinement
   mqp_host::DevBuf def1, def2;  // deformed images of the deforming refinement
   mqp_host::DevBuf huge;        // scratch slots of the 2D kernel for search windows above 128

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "mqp_finish.cuh"
 #include "mqp_internal.h"
 
 namespace mqp {
@@ -260,6 +261,62 @@ size_t integral2d_scratch_bytes(int H, int W) {  // chunk totals and their runni
 
 size_t integral3d_scratch_bytes(int H, int W, int D) {
   return integral2d_scratch_bytes(H, W) * (size_t)(D < 65535 ? D : 65535);
+}
+
+// ---------------------------------------------------------------------------
+// window-sum map of a pass (mqp_finish.cuh) from the integral image of img2^2
+// ---------------------------------------------------------------------------
+// One thread per row of the map and WMAP columns: consecutive threads read
+// and write consecutive rows.
+constexpr int WMAP = 4;
+
+__global__ void __launch_bounds__(256) window_map_kernel(const double* __restrict__ II, int H, int W, int IS1, int IS2,
+                                                         int SM1, int SM2, float2* __restrict__ ws,
+                                                         double* __restrict__ wd, int ldw, int cols, int col0) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= ldw) return;
+  const long long ld = (long long)H + 1;
+  const int i = k - SM1;
+  const int r0 = i > 0 ? i : 0, r1 = i + IS1 < H ? i + IS1 : H;
+  const int j0 = col0 + (int)blockIdx.y * WMAP;
+  double a11[WMAP], a10[WMAP], a01[WMAP], a00[WMAP];
+#pragma unroll
+  for (int t = 0; t < WMAP; ++t) {
+    const int j = j0 + t - SM2;
+    const int c0 = j > 0 ? j : 0, c1 = j + IS2 < W ? j + IS2 : W;
+    const bool any = j0 + t < cols && r1 > r0 && c1 > c0;
+    const double* A1 = II + ld * c1;
+    const double* A0 = II + ld * c0;
+    a11[t] = any ? A1[r1] : 0.0;
+    a10[t] = any ? A1[r0] : 0.0;
+    a01[t] = any ? A0[r1] : 0.0;
+    a00[t] = any ? A0[r0] : 0.0;
+  }
+#pragma unroll
+  for (int t = 0; t < WMAP; ++t) {
+    if (j0 + t < cols) {
+      const double S2 = (a11[t] - a10[t]) - (a01[t] - a00[t]);  // box_sum's order
+      const float s = (float)S2;
+      ws[k + (long long)ldw * (j0 + t)] = make_float2(s, sqrtf(s));
+      if (wd) wd[k + (long long)ldw * (j0 + t)] = S2;
+    }
+  }
+}
+
+size_t window_map_bytes(int H, int W, int IS1, int IS2, int SM1, int SM2) {
+  return (size_t)winmap_ld(H, IS1, SM1) * (size_t)winmap_ld(W, IS2, SM2) * sizeof(float2);
+}
+
+cudaError_t launch_window_map(const double* II, int H, int W, int IS1, int IS2, int SM1, int SM2, float2* ws,
+                              double* wd, int m0, int m1, cudaStream_t s) {
+  const int ldw = winmap_ld(H, IS1, SM1);
+  const int threads = ldw < 256 ? (ldw + 31) / 32 * 32 : 256;
+  for (int c0 = m0; c0 < m1; c0 += 65535 * WMAP) {
+    const int n = m1 - c0 < 65535 * WMAP ? m1 - c0 : 65535 * WMAP;
+    const dim3 grid((ldw + threads - 1) / threads, (n + WMAP - 1) / WMAP);
+    window_map_kernel<<<grid, threads, 0, s>>>(II, H, W, IS1, IS2, SM1, SM2, ws, wd, ldw, c0 + n, c0);
+  }
+  return cudaGetLastError();
 }
 
 }  // namespace mqp

@@ -26,6 +26,17 @@ cudaError_t launch_integral2d_cols(const void* img, int dtype, int H, int W, int
                                    double* out, double* scratch, cudaStream_t s);
 size_t integral2d_scratch_bytes(int H, int W);
 
+// The window-sum map of a pass (Piv2dArgs::ws, mqp_finish.cuh) from the
+// integral image of img2^2; ws holds window_map_bytes(...) bytes, and wd
+// (the sums in FP64, or null) as many.  Columns
+// [m0, m1) of the map (winmap_ld(W, IS2, SM2) in all): column m reads integral
+// columns up to m - SM2 + IS2.
+size_t window_map_bytes(int H, int W, int IS1, int IS2, int SM1, int SM2);
+cudaError_t launch_window_map(const double* II, int H, int W, int IS1, int IS2, int SM1, int SM2, float2* ws,
+                              double* wd, int m0, int m1, cudaStream_t s);
+// passes whose kernel takes the map
+bool piv2d_takes_map(int IS1, int IS2, int SM1, int SM2, int alg, bool SN);
+
 // The same for a column-major H x W x D volume: out is (H+1) x (W+1) x (D+1),
 // first plane zero; scratch holds integral3d_scratch_bytes(H, W, D) bytes.
 cudaError_t launch_integral3d(const void* img, int dtype, int H, int W, int D, bool square,
@@ -48,6 +59,11 @@ cudaError_t launch_piv2d_w64(const Piv2dArgs& a, int alg, bool prune, cudaStream
 cudaError_t launch_piv2d_w32(const Piv2dArgs& a, int alg, bool prune, cudaStream_t s, std::string& err);
 cudaError_t launch_piv2d_b64(const Piv2dBatch& b, cudaStream_t s, std::string& err);
 cudaError_t launch_piv2d_b32(const Piv2dBatch& b, cudaStream_t s, std::string& err);
+
+// Strip kernel (mqp_piv2d_strip.cu): FFTCC / NSQECC passes of whole IA columns
+// without a predictor, whose IAs share their windows' row transforms.
+bool piv2d_strip_ok(const Piv2dArgs& a, int alg);
+cudaError_t launch_piv2d_strip(const Piv2dArgs& a, int alg, cudaStream_t s, std::string& err);
 
 // One persistent launch of the fused 2D kernel over the IAs of many image
 // pairs that share a kernel variant (N, prune, alg, dtype): items[k] (device

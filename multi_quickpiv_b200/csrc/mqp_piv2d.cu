@@ -105,12 +105,19 @@ cudaError_t launch_piv2d_batch(const Piv2dBatch& b, cudaStream_t s, std::string&
   return cudaErrorInvalidValue;
 }
 
+bool piv2d_takes_map(int IS1, int IS2, int SM1, int SM2, int alg, bool SN) {
+  (void)SN;
+  return alg == ALG_NSQECC && !direct2d_ok(IS1, IS2, SM1, SM2) && piv2d_fft_len(IS1 + 2 * SM1, IS2 + 2 * SM2) == 64 &&
+         IS1 <= 32 && IS2 <= 32;
+}
+
 cudaError_t launch_piv2d(const Piv2dArgs& a, int alg, cudaStream_t s, std::string& err) {
   if (direct2d_ok(a.IS1, a.IS2, a.SM1, a.SM2)) return launch_piv2d_direct(a, alg, s, err);
   const int SS1 = a.IS1 + 2 * a.SM1, SS2 = a.IS2 + 2 * a.SM2;
   const int N = piv2d_fft_len(SS1, SS2);
   const bool prune = (a.IS1 <= N / 2) && (a.IS2 <= N / 2);
   if (piv2d_team_ok(N, prune, alg)) return launch_piv2d_team(a, N, alg, s, err);
+  if (piv2d_strip_ok(a, alg)) return launch_piv2d_strip(a, alg, s, err);
   if (N == 64) return launch_piv2d_w64(a, alg, prune, s, err);
   if (N == 32) return launch_piv2d_w32(a, alg, prune, s, err);
   if (N == 128) return launch_piv2d_big(a, alg, s, err);

@@ -58,6 +58,9 @@ struct Piv2dArgs {
   int computeSN;
   int* status;           // device error flag (non-zero = failure), or null
   float2* huge;          // FFT length 256 (mqp_piv2d_huge.cuh): one scratch slot per resident block
+  const float2* ws;      // window-sum map of img2^2 (mqp_finish.cuh), or null: read the integral image
+  const double* wd;      // SN passes: the map's sums in FP64
+  int ldw;               // their column length
 };
 
 // Geometry of one IA in pad coordinates (0-based).  Pad index p along an
