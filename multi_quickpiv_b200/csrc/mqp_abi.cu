@@ -122,18 +122,21 @@ static int integrals_2d(mqp_ctx* ctx, const Problem& pb, const void* d1, const v
 // The window-sum map of a 2D pass that takes one (ctx buffer), after the
 // integral columns of image columns [0, x1): map columns [*m0, ...) as far as
 // those go; *m0 moves on.
-static int window_map_2d(mqp_ctx* ctx, const Problem& pb, bool SN, cudaStream_t s, int x1, int* m0) {
-  if (!mqp::piv2d_takes_map(pb.IS[0], pb.IS[1], pb.SM[0], pb.SM[1], pb.alg, SN)) return MQP_OK;
+static int window_map_2d(mqp_ctx* ctx, const Problem& pb, bool SN, bool pred, cudaStream_t s, int x1, int* m0) {
+  if (!mqp::piv2d_takes_map(pb.IS[0], pb.IS[1], pb.SM[0], pb.SM[1], pb.alg, SN, pred)) return MQP_OK;
   const int H = (int)pb.dims[0], W = (int)pb.dims[1];
-  const size_t mb = mqp::window_map_bytes(H, W, pb.IS[0], pb.IS[1], pb.SM[0], pb.SM[1]);
-  cudaError_t e = ctx->wmap.ensure(SN ? 2 * mb : mb);  // SN: the FP64 sums follow
+  auto layout = [&](void* base) { return mqp::window_map(H, W, pb.IS[0], pb.IS[1], pb.SM[0], pb.SM[1], pb.alg, SN, base); };
+  cudaError_t e = ctx->wmap.ensure(layout(nullptr).bytes);
+  if (e == cudaErrorMemoryAllocation) {  // the kernels read the integral images instead
+    cudaGetLastError();
+    return MQP_OK;
+  }
   if (e != cudaSuccess) return cuda_fail(ctx, e, "window-sum map");
-  const int cols = mqp::winmap_ld(W, pb.IS[1], pb.SM[1]);
-  const int m1 = x1 == W ? cols : std::min(cols, std::max(*m0, x1 - pb.IS[1] + pb.SM[1] + 1));
+  const mqp::WindowMap m = layout(ctx->wmap.ptr);
+  const int m1 = x1 == W ? m.cols : std::min(m.cols, std::max(*m0, x1 - pb.IS[1] + pb.SM[1] + 1));
   ProfileScope ps(ctx, s, 0, 0);
-  if (m1 > *m0 && (e = mqp::launch_window_map((const double*)ctx->IIg2.ptr, H, W, pb.IS[0], pb.IS[1], pb.SM[0], pb.SM[1],
-                                              (float2*)ctx->wmap.ptr, SN ? (double*)((char*)ctx->wmap.ptr + mb) : nullptr, *m0,
-                                              m1, s)) != cudaSuccess)
+  if (m1 > *m0 && (e = mqp::launch_window_map((const double*)ctx->IIg2.ptr, (const double*)ctx->IIg.ptr, H, W, pb.IS[0],
+                                              pb.IS[1], pb.SM[0], pb.SM[1], m, *m0, m1, s)) != cudaSuccess)
     return cuda_fail(ctx, e, "window-sum map");
   *m0 = m1;
   return MQP_OK;
@@ -157,12 +160,15 @@ static mqp::Piv2dArgs args_2d(mqp_ctx* ctx, const Problem& pb, const mqp_params*
     a.IIg = (const double*)ctx->IIg.ptr;
     a.II1 = (const double*)ctx->II1.ptr;
   }
-  if (mqp::piv2d_takes_map(pb.IS[0], pb.IS[1], pb.SM[0], pb.SM[1], pb.alg, dSN != nullptr)) {
-    a.ws = (const float2*)ctx->wmap.ptr;
-    if (dSN)
-      a.wd = (const double*)((const char*)ctx->wmap.ptr + mqp::window_map_bytes((int)pb.dims[0], (int)pb.dims[1], pb.IS[0],
-                                                                                pb.IS[1], pb.SM[0], pb.SM[1]));
-    a.ldw = mqp::winmap_ld((int)pb.dims[0], pb.IS[0], pb.SM[0]);
+  if (mqp::piv2d_takes_map(pb.IS[0], pb.IS[1], pb.SM[0], pb.SM[1], pb.alg, dSN != nullptr, dpred != nullptr)) {
+    const mqp::WindowMap m = mqp::window_map((int)pb.dims[0], (int)pb.dims[1], pb.IS[0], pb.IS[1], pb.SM[0], pb.SM[1],
+                                             pb.alg, dSN != nullptr, ctx->wmap.ptr);
+    if (ctx->wmap.bytes >= m.bytes) {
+      a.ws = m.ws;
+      a.wd = m.wd;
+      a.wz = m.wz;
+      a.ldw = m.ldw;
+    }
   }
   a.pred = dpred;
   a.VF = dVF;
@@ -211,7 +217,7 @@ int run_pass_2d(mqp_ctx* ctx, const Problem& pb, const mqp_params* p, const void
   int rc = integrals_2d(ctx, pb, d1, d2, dtype, s, 0, W);
   if (rc != MQP_OK) return rc;
   int m0 = 0;
-  if ((rc = window_map_2d(ctx, pb, dSN != nullptr, s, W, &m0)) != MQP_OK) return rc;
+  if ((rc = window_map_2d(ctx, pb, dSN != nullptr, dpred != nullptr, s, W, &m0)) != MQP_OK) return rc;
   mqp::Piv2dArgs a = args_2d(ctx, pb, p, d1, d2, dmask, dskip, dtype, dVF, dSN, dpred, dplanes, ia_begin, ia_end);
   if (huge) {
     cudaError_t e = ctx->huge.ensure(mqp::piv2d_huge_scratch_bytes(ctx->device, 2 * pb.SM[0] + 1, 2 * pb.SM[1] + 1));
@@ -533,7 +539,7 @@ static int host_pipelined_2d(mqp_ctx* ctx, const Problem& pb, const mqp_params* 
       return cuda_fail(ctx, e, "pipeline order");
     int rc = integrals_2d(ctx, pb, ctx->img1.ptr, ctx->img2.ptr, dtype, s, x0, x1);
     if (rc != MQP_OK) return rc;
-    if ((rc = window_map_2d(ctx, pb, dSN != nullptr, s, x1, &m0)) != MQP_OK) return rc;
+    if ((rc = window_map_2d(ctx, pb, dSN != nullptr, false, s, x1, &m0)) != MQP_OK) return rc;
     int64_t c1 = done_cols;
     while (c1 < vf2 && (x1 == W || need(c1) <= x1)) ++c1;
     if (c1 > done_cols) {

@@ -37,6 +37,8 @@ constexpr float PEAK_GAP = 1e-5f;
 // (integral-image differences in box_sum's order), for i in [-SM1, H - IS1 +
 // SM1] and j likewise: one 8-byte read per lag instead of four FP64 reads, and
 // the square root once per window position instead of once per lag and IA.
+// ZNCC: wz holds the FP64 sums of img2^2 and img2 (the variance about the search
+// mean cancels), one 16-byte read instead of eight of 8 bytes.
 MQP_HD MQP_FI int winmap_ld(int H, int IS, int SM) { return H - IS + 2 * SM + 1; }
 
 // Last lag along an axis whose window sum is the map's: windows clip at the
@@ -95,86 +97,240 @@ __device__ __forceinline__ void unmapped_lags(const LagRanges& R, int e1, int e2
   }
 }
 
-// Lag box walk of one warp.  cc(s1, s2) is the raw correlation before the
-// transforms' scale; rows s1 < lane_rows go one per lane (s1 = lane + 32 k),
-// the others lanes over s2.  Returns the first maximum > 0 in column-major
-// order (bidx = s1 + P1 s2, -1 = none), on every lane.
-template <int ALG, typename CC>
+__device__ __forceinline__ float sqrt_approx(float x) {
+#if defined(__CUDA_ARCH__)
+  float r;
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+#else
+  return sqrtf(x);
+#endif
+}
+
+// Lag box walk of NT threads (one warp, or a block whose every thread calls
+// it).  cc(s1, s2) * scale is the raw correlation.  Returns the first maximum > 0
+// in column-major order (bidx = s1 + P1 s2, -1 = none) on every thread.  Window
+// sums come from the pass's map (a.ws, ZNCC: a.wz), from the on-chip table lw
+// (LWN = N, mqp_piv2d.cuh) or, without either, from the integral images.  red:
+// 2 NT / 32 doubles of shared memory when NT > 32 (the caller's barriers
+// around it).
+template <int ALG, int NT, int LWN, typename CC>
 __device__ __forceinline__ int finish_search(const Piv2dArgs& a, const IAGeom& g, const IAScalars& sc,
-                                             const LagRanges& R, int lane, int lane_rows, int P1, double scale,
-                                             CC cc) {
+                                             const LagRanges& R, int tid, int P1, double scale, CC cc,
+                                             const double* lw, double* red) {
   const unsigned FULL = 0xffffffffu;
+  static_assert(ALG == ALG_FFTCC || ALG == ALG_ZNCC || ALG == ALG_NSQECC, "unmasked similarities");
   const float sqF = sqrtf((float)sc.sumF2), F2 = (float)sc.sumF2;
-  const float m2 = -2.f * (float)scale;
+  const float fscale = (float)scale, m2 = -2.f * fscale;
   TopTwo t;
   t.b1 = t.b2 = 0.f;
   t.idx = -1;
-  bool full = false;  // every lag of the box in full
-  if (ALG == ALG_FFTCC) {
-    for (int s1 = lane; s1 < lane_rows; s1 += 32)
-      if (s1 >= R.lo1 && s1 <= R.hi1) {
-#pragma unroll 4
-        for (int s2 = R.lo2; s2 <= R.hi2; ++s2) first_take(t, cc(s1, s2), s1 + P1 * s2);
+  // every lag of the box in full: also where the approximations could leave
+  // the normal FP32 range
+  const bool full = ALG != ALG_FFTCC && !(sc.sumF2 > 1e-30 && sc.sumF2 < 1e30);
+  const bool map = ALG == ALG_NSQECC ? a.ws != nullptr : (ALG == ALG_ZNCC && !LWN && a.wz != nullptr);
+  int e1 = R.hi1, e2 = R.hi2;
+  if (map) {
+    e1 = min(e1, lag_mapped_max(a.SM1, a.IS1, g.g01, g.hi1, a.H));
+    e2 = min(e2, lag_mapped_max(a.SM2, a.IS2, g.g02, g.hi2, a.W));
+  }
+  // lag q of the walk: s1 = lo1 + q % w1, s2 = lo2 + q / w1, so that a warp
+  // reads runs of consecutive rows
+  const int w1 = e1 - R.lo1 + 1, total = w1 > 0 && e2 >= R.lo2 ? w1 * (e2 - R.lo2 + 1) : 0;
+  if (!full && total > 0) {
+    const int d2 = NT / w1, d1 = NT - d2 * w1;
+    int s2 = R.lo2 + tid / w1, s1 = R.lo1 + tid % w1;
+    auto step = [&]() {
+      s1 += d1;
+      s2 += d2;
+      if (s1 > e1) {
+        s1 -= w1;
+        ++s2;
       }
-    for (int s1 = lane_rows > R.lo1 ? lane_rows : R.lo1; s1 <= R.hi1; ++s1)
-      for (int s2 = R.lo2 + lane; s2 <= R.hi2; s2 += 32) first_take(t, cc(s1, s2), s1 + P1 * s2);
-  } else {
-    // outside this range the approximations could leave the normal FP32 range
-    full = !(sc.sumF2 > 1e-30 && sc.sumF2 < 1e30);
-    const int m1 = lag_mapped_max(a.SM1, a.IS1, g.g01, g.hi1, a.H), e1 = m1 < R.hi1 ? m1 : R.hi1;
-    const int m2l = lag_mapped_max(a.SM2, a.IS2, g.g02, g.hi2, a.W), e2 = m2l < R.hi2 ? m2l : R.hi2;
-    const float2* w0 = a.ws + (g.g01 + a.SM1) + (long long)a.ldw * (g.g02 + a.SM2);
-    auto value = [&](float2 w, float c) {
-      const float d = w.y * sqF;
-      const float n = fmaf(m2, c, F2 + w.x);
-      return d * rcp_approx(n + d);
     };
-    if (!full) {
-      for (int s1 = lane; s1 < lane_rows; s1 += 32)
-        if (s1 >= R.lo1 && s1 <= e1) {
-          for (int b = R.lo2; b <= e2; b += 8) {
-            float2 q[8];
+    if (ALG == ALG_FFTCC) {
+#pragma unroll 4
+      for (int q = tid; q < total; q += NT) {
+        first_take(t, cc(s1, s2), s1 + P1 * s2);
+        step();
+      }
+    } else {
+      // B lags' correlations and sums (load) are read before any is used (value)
+      auto walk = [&](auto load, auto value) {
+        constexpr int B = 8;
+        if (NT == 32 && w1 > 20) {
+          // most of a warp's lanes find a row of their own: no index to keep per lag
+          const int s1 = min(R.lo1 + tid, e1);
+          const bool mine = R.lo1 + tid <= e1;
+#pragma unroll 1
+          for (int b = R.lo2; b <= e2; b += B) {
+            decltype(load(0, 0)) m[B];
 #pragma unroll
-            for (int k = 0; k < 8; ++k)  // past the box: its last column again, not taken
-              q[k] = __ldg(w0 + s1 + (long long)a.ldw * min(b + k, e2));
+            for (int k = 0; k < B; ++k) m[k] = load(s1, min(b + k, e2));
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-              const float v = value(q[k], cc(s1, min(b + k, e2)));
-              if (b + k <= e2) top_take(t, v, s1 + P1 * (b + k));
+            for (int k = 0; k < B; ++k) {
+              const float v = value(m[k], cc(s1, min(b + k, e2)));
+              if (mine && b + k <= e2) top_take(t, v, s1 + P1 * (b + k));
             }
           }
+#pragma unroll 1
+          for (int u1 = R.lo1 + 32; u1 <= e1; ++u1)  // rows past the lanes, lanes over columns
+            for (int u2 = R.lo2 + tid; u2 <= e2; u2 += 32) top_take(t, value(load(u1, u2), cc(u1, u2)), u1 + P1 * u2);
+          return;
         }
-      for (int s1 = lane_rows > R.lo1 ? lane_rows : R.lo1; s1 <= e1; ++s1)
-        for (int s2 = R.lo2 + lane; s2 <= e2; s2 += 32)
-          top_take(t, value(__ldg(w0 + s1 + (long long)a.ldw * s2), cc(s1, s2)), s1 + P1 * s2);
-      unmapped_lags(R, e1, e2, lane, [&](int s1, int s2) {
-        top_take(t, (float)finish_one<ALG>(a, g, sc, s1, s2, (double)cc(s1, s2) * scale), s1 + P1 * s2);
-      });
+#pragma unroll 1
+        for (int q = tid; q < total; q += NT * B) {
+          decltype(load(0, 0)) m[B];
+          float c[B];
+          int id[B];
+#pragma unroll
+          for (int k = 0; k < B; ++k) {
+            const bool in = q + k * NT < total;
+            id[k] = in ? s1 + P1 * s2 : -1;
+            const int u1 = in ? s1 : R.lo1, u2 = in ? s2 : R.lo2;  // past the box: its first lag, not taken
+            c[k] = cc(u1, u2);
+            m[k] = load(u1, u2);
+            step();
+          }
+#pragma unroll
+          for (int k = 0; k < B; ++k) {
+            const float v = value(m[k], c[k]);
+            if (id[k] >= 0) top_take(t, v, id[k]);
+          }
+        }
+      };
+      auto nsqecc = [&](float s, float q, float c) {
+        const float d = q * sqF;
+        return d * rcp_approx(fmaf(m2, c, F2 + s) + d);
+      };
+      auto zncc = [&](double S2, double S1, double n, float c) {
+        const double SG = S2 - 2.0 * sc.meanG * S1 + n * sc.meanG * sc.meanG;
+        return c * fscale * rsqrtf((float)(SG > 0.0 ? SG : 0.0));
+      };
+      const long long w0 = (g.g01 + a.SM1) + (long long)a.ldw * (g.g02 + a.SM2);
+      auto window = [&](int u1, int u2, int& r0, int& r1, int& c0, int& c1) {
+        lag_window(u1, a.IS1, g.g01, g.lo1, g.hi1, r0, r1);
+        lag_window(u2, a.IS2, g.g02, g.lo2, g.hi2, c0, c1);
+      };
+      if (LWN) {
+        walk([&](int u1, int u2) { return lw[lw_at(LWN, u1, u2)]; },
+             [&](double S2, float c) { return c * fscale * rsqrtf((float)S2); });
+      } else if (ALG == ALG_NSQECC && map) {
+        const float2* w = a.ws + w0;
+        walk([&](int u1, int u2) { return __ldg(w + (u1 + (long long)a.ldw * u2)); },
+             [&](float2 m, float c) { return nsqecc(m.x, m.y, c); });
+      } else if (ALG == ALG_NSQECC) {
+        walk(
+            [&](int u1, int u2) {
+              int r0, r1, c0, c1;
+              window(u1, u2, r0, r1, c0, c1);
+              return box_sum(a.IIg2, a.H, r0, r1, c0, c1);
+            },
+            [&](double S2, float c) { return nsqecc((float)S2, sqrt_approx((float)S2), c); });
+      } else if (map) {
+        const double2* w = a.wz + w0;
+        // interrogation-sized windows, but for those the image's edge cuts
+        const double nw = (double)a.IS1 * (double)a.IS2;
+        const bool whole = g.g01 + R.lo1 >= 0 && g.g01 + e1 + a.IS1 <= a.H && g.g02 + R.lo2 >= 0 && g.g02 + e2 + a.IS2 <= a.W;
+        walk(
+            [&](int u1, int u2) {
+              const double2 v = __ldg(w + (u1 + (long long)a.ldw * u2));
+              double n = nw;
+              if (!whole) {
+                int r0, r1, c0, c1;
+                window(u1, u2, r0, r1, c0, c1);
+                n = (double)(r1 - r0) * (double)(c1 - c0);
+              }
+              return make_double3(v.x, v.y, n);
+            },
+            [&](double3 m, float c) { return zncc(m.x, m.y, m.z, c); });
+      } else {
+        walk(
+            [&](int u1, int u2) {
+              int r0, r1, c0, c1;
+              window(u1, u2, r0, r1, c0, c1);
+              return make_double3(box_sum(a.IIg2, a.H, r0, r1, c0, c1), box_sum(a.IIg, a.H, r0, r1, c0, c1),
+                                  (double)(r1 - r0) * (double)(c1 - c0));
+            },
+            [&](double3 m, float c) { return zncc(m.x, m.y, m.z, c); });
+      }
+    }
+  }
+  if (!full && map) {
+    // the lags the map does not hold: rows past e1, then columns past e2
+    const int w2 = R.hi2 - R.lo2 + 1, nr = R.hi1 > e1 ? (R.hi1 - max(e1, R.lo1 - 1)) * w2 : 0;
+    const int h1 = e1 - R.lo1 + 1, nc = R.hi2 > e2 && h1 > 0 ? (R.hi2 - max(e2, R.lo2 - 1)) * h1 : 0;
+#pragma unroll 1
+    for (int q = tid; q < nr + nc; q += NT) {
+      const int s1 = q < nr ? R.hi1 - q / w2 : R.lo1 + (q - nr) % h1;
+      const int s2 = q < nr ? R.lo2 + q % w2 : R.hi2 - (q - nr) / h1;
+      const float v = (float)finish_one<ALG>(a, g, sc, s1, s2, (double)cc(s1, s2) * scale);
+      top_take(t, ALG == ALG_ZNCC ? v * sqF : v, s1 + P1 * s2);  // on the walk's scale
     }
   }
   // the largest value of the box, and what comes within the gap of it
+  float* redf = reinterpret_cast<float*>(red);
+  const int warp = tid >> 5, lane = tid & 31;
+  constexpr int NW = NT / 32;
   float mx = t.b1;
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(FULL, mx, off));
+  if (NT > 32) {
+    if (lane == 0) redf[warp] = mx;
+    __syncthreads();
+    mx = redf[0];
+    for (int w = 1; w < NW; ++w) mx = fmaxf(mx, redf[w]);
+    __syncthreads();
+  }
   if (!full) {
     if (!(mx > 0.f)) return -1;
     if (ALG == ALG_FFTCC) {  // exact values: the first of equal maxima
       int idx = t.b1 == mx ? t.idx : 0x7fffffff;
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) idx = min(idx, __shfl_xor_sync(FULL, idx, off));
+      if (NT > 32) {
+        int* ri = reinterpret_cast<int*>(red);
+        if (lane == 0) ri[warp] = idx;
+        __syncthreads();
+        idx = ri[0];
+        for (int w = 1; w < NW; ++w) idx = min(idx, ri[w]);
+        __syncthreads();
+      }
       return idx;
     }
     const float th = mx * (1.f - PEAK_GAP);
-    const unsigned near = __ballot_sync(FULL, t.b1 >= th);
-    if (__popc(near) == 1 && !__any_sync(FULL, t.b2 >= th)) return __shfl_sync(FULL, t.idx, __ffs(near) - 1);
+    // how many threads hold a value within the gap (one that holds two counts
+    // as two), and the lag of the only one
+    int cnt = (t.b1 >= th) + (t.b2 >= th), idx = t.b1 >= th ? t.idx : -1;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      cnt += __shfl_xor_sync(FULL, cnt, off);
+      idx = max(idx, __shfl_xor_sync(FULL, idx, off));
+    }
+    if (NT > 32) {
+      int* ri = reinterpret_cast<int*>(red);
+      if (lane == 0) {
+        ri[2 * warp] = cnt;
+        ri[2 * warp + 1] = idx;
+      }
+      __syncthreads();
+      cnt = ri[0];
+      idx = ri[1];
+      for (int w = 1; w < NW; ++w) {
+        cnt += ri[2 * w];
+        idx = max(idx, ri[2 * w + 1]);
+      }
+      __syncthreads();
+    }
+    if (cnt == 1) return idx;
   }
   double best = 0.0;
   int bidx = -1;
-  const int w2 = R.hi2 - R.lo2 + 1, total = (R.hi1 - R.lo1 + 1) * w2;
+  const int w2 = R.hi2 - R.lo2 + 1, all = (R.hi1 - R.lo1 + 1) * w2;
 #pragma unroll 1
-  for (int q = lane; q < total; q += 32) {
+  for (int q = tid; q < all; q += NT) {
     const int s1 = R.lo1 + q / w2, s2 = R.lo2 + q % w2;
-    peak_take(finish_one<ALG>(a, g, sc, s1, s2, (double)cc(s1, s2) * scale), s1 + P1 * s2, best, bidx);
+    peak_take(finish_one<ALG, LWN>(a, g, sc, s1, s2, (double)cc(s1, s2) * scale, 0.0, lw), s1 + P1 * s2, best, bidx);
   }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) {
@@ -182,14 +338,28 @@ __device__ __forceinline__ int finish_search(const Piv2dArgs& a, const IAGeom& g
     const int oi = __shfl_xor_sync(FULL, bidx, off);
     peak_merge(best, bidx, ob, oi);
   }
+  if (NT > 32) {
+    if (lane == 0) {
+      red[2 * warp] = best;
+      red[2 * warp + 1] = (double)bidx;
+    }
+    __syncthreads();
+    best = red[0];
+    bidx = (int)red[1];
+    for (int w = 1; w < NW; ++w) peak_merge(best, bidx, red[2 * w], (int)red[2 * w + 1]);
+    __syncthreads();
+  }
   return bidx;
 }
 
+// Whether an unmasked pass ends in finish_search.
+MQP_HD MQP_FI bool finish_fast(const Piv2dArgs& a) { return a.SN == nullptr && a.planes == nullptr; }
+
 // refine2d_warp from the raw correlations: nine lanes evaluate the 3x3
 // neighbourhood of the peak (p1, p2) in full.
-template <int ALG, typename CC>
+template <int ALG, int LWN, typename CC>
 __device__ __forceinline__ void finish_refine(const Piv2dArgs& a, const IAGeom& g, const IAScalars& sc, int p1, int p2,
-                                              int lane, double scale, CC cc, double& r1, double& r2) {
+                                              int lane, double scale, CC cc, const double* lw, double& r1, double& r2) {
   const unsigned FULL = 0xffffffffu;
   r1 = p1;
   r2 = p2;
@@ -200,7 +370,7 @@ __device__ __forceinline__ void finish_refine(const Piv2dArgs& a, const IAGeom& 
   double v = 0.0;
   if (lane < 9) {
     const int s1 = p1 - 1 + lane % 3, s2 = p2 - 1 + lane / 3;
-    v = finish_one<ALG>(a, g, sc, s1, s2, (double)cc(s1, s2) * scale);
+    v = finish_one<ALG, LWN>(a, g, sc, s1, s2, (double)cc(s1, s2) * scale, 0.0, lw);
   }
   double mn = __shfl_sync(FULL, v, 0);
 #pragma unroll

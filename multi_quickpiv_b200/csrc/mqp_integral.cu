@@ -270,15 +270,8 @@ size_t integral3d_scratch_bytes(int H, int W, int D) {
 // and write consecutive rows.
 constexpr int WMAP = 4;
 
-__global__ void __launch_bounds__(256) window_map_kernel(const double* __restrict__ II, int H, int W, int IS1, int IS2,
-                                                         int SM1, int SM2, float2* __restrict__ ws,
-                                                         double* __restrict__ wd, int ldw, int cols, int col0) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= ldw) return;
-  const long long ld = (long long)H + 1;
-  const int i = k - SM1;
-  const int r0 = i > 0 ? i : 0, r1 = i + IS1 < H ? i + IS1 : H;
-  const int j0 = col0 + (int)blockIdx.y * WMAP;
+__device__ __forceinline__ void window_sums(const double* __restrict__ II, long long ld, int W, int IS2, int SM2, int r0,
+                                            int r1, int j0, int cols, double (&S)[WMAP]) {
   double a11[WMAP], a10[WMAP], a01[WMAP], a00[WMAP];
 #pragma unroll
   for (int t = 0; t < WMAP; ++t) {
@@ -293,28 +286,63 @@ __global__ void __launch_bounds__(256) window_map_kernel(const double* __restric
     a00[t] = any ? A0[r0] : 0.0;
   }
 #pragma unroll
+  for (int t = 0; t < WMAP; ++t) S[t] = (a11[t] - a10[t]) - (a01[t] - a00[t]);  // box_sum's order
+}
+
+// NSQECC: ws (and wd) from II2; ZNCC: wz from II2 and II1 (IIg2 and IIg).
+__global__ void __launch_bounds__(256) window_map_kernel(const double* __restrict__ II2, const double* __restrict__ II1,
+                                                         int H, int W, int IS1, int IS2, int SM1, int SM2,
+                                                         WindowMap m, int cols, int col0) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= m.ldw) return;
+  const long long ld = (long long)H + 1;
+  const int i = k - SM1;
+  const int r0 = i > 0 ? i : 0, r1 = i + IS1 < H ? i + IS1 : H;
+  const int j0 = col0 + (int)blockIdx.y * WMAP;
+  double S2[WMAP], S1[WMAP];
+  window_sums(II2, ld, W, IS2, SM2, r0, r1, j0, cols, S2);
+  if (m.wz) window_sums(II1, ld, W, IS2, SM2, r0, r1, j0, cols, S1);
+#pragma unroll
   for (int t = 0; t < WMAP; ++t) {
     if (j0 + t < cols) {
-      const double S2 = (a11[t] - a10[t]) - (a01[t] - a00[t]);  // box_sum's order
-      const float s = (float)S2;
-      ws[k + (long long)ldw * (j0 + t)] = make_float2(s, sqrtf(s));
-      if (wd) wd[k + (long long)ldw * (j0 + t)] = S2;
+      const long long at = k + (long long)m.ldw * (j0 + t);
+      if (m.wz) {
+        m.wz[at] = make_double2(S2[t], S1[t]);
+      } else {
+        const float s = (float)S2[t];
+        m.ws[at] = make_float2(s, sqrtf(s));
+        if (m.wd) m.wd[at] = S2[t];
+      }
     }
   }
 }
 
-size_t window_map_bytes(int H, int W, int IS1, int IS2, int SM1, int SM2) {
-  return (size_t)winmap_ld(H, IS1, SM1) * (size_t)winmap_ld(W, IS2, SM2) * sizeof(float2);
+WindowMap window_map(int H, int W, int IS1, int IS2, int SM1, int SM2, int alg, bool SN, void* base) {
+  WindowMap m;
+  m.ldw = winmap_ld(H, IS1, SM1);
+  m.cols = winmap_ld(W, IS2, SM2);
+  const size_t n = (size_t)m.ldw * (size_t)m.cols;
+  if (alg == ALG_ZNCC) {
+    m.wz = (double2*)base;
+    m.bytes = n * sizeof(double2);
+  } else {
+    m.ws = (float2*)base;
+    m.bytes = n * sizeof(float2);
+    if (SN) {
+      m.wd = (double*)((char*)base + m.bytes);
+      m.bytes += n * sizeof(double);
+    }
+  }
+  return m;
 }
 
-cudaError_t launch_window_map(const double* II, int H, int W, int IS1, int IS2, int SM1, int SM2, float2* ws,
-                              double* wd, int m0, int m1, cudaStream_t s) {
-  const int ldw = winmap_ld(H, IS1, SM1);
-  const int threads = ldw < 256 ? (ldw + 31) / 32 * 32 : 256;
+cudaError_t launch_window_map(const double* II2, const double* II1, int H, int W, int IS1, int IS2, int SM1, int SM2,
+                              const WindowMap& m, int m0, int m1, cudaStream_t s) {
+  const int threads = m.ldw < 256 ? (m.ldw + 31) / 32 * 32 : 256;
   for (int c0 = m0; c0 < m1; c0 += 65535 * WMAP) {
     const int n = m1 - c0 < 65535 * WMAP ? m1 - c0 : 65535 * WMAP;
-    const dim3 grid((ldw + threads - 1) / threads, (n + WMAP - 1) / WMAP);
-    window_map_kernel<<<grid, threads, 0, s>>>(II, H, W, IS1, IS2, SM1, SM2, ws, wd, ldw, c0 + n, c0);
+    const dim3 grid((m.ldw + threads - 1) / threads, (n + WMAP - 1) / WMAP);
+    window_map_kernel<<<grid, threads, 0, s>>>(II2, II1, H, W, IS1, IS2, SM1, SM2, m, c0 + n, c0);
   }
   return cudaGetLastError();
 }

@@ -26,16 +26,22 @@ cudaError_t launch_integral2d_cols(const void* img, int dtype, int H, int W, int
                                    double* out, double* scratch, cudaStream_t s);
 size_t integral2d_scratch_bytes(int H, int W);
 
-// The window-sum map of a pass (Piv2dArgs::ws, mqp_finish.cuh) from the
-// integral image of img2^2; ws holds window_map_bytes(...) bytes, and wd
-// (the sums in FP64, or null) as many.  Columns
-// [m0, m1) of the map (winmap_ld(W, IS2, SM2) in all): column m reads integral
-// columns up to m - SM2 + IS2.
-size_t window_map_bytes(int H, int W, int IS1, int IS2, int SM1, int SM2);
-cudaError_t launch_window_map(const double* II, int H, int W, int IS1, int IS2, int SM1, int SM2, float2* ws,
-                              double* wd, int m0, int m1, cudaStream_t s);
+// The window-sum map of a pass (Piv2dArgs::ws / wd / wz, mqp_finish.cuh) over
+// `bytes` of device memory at `base`, filled from the integral images of img2^2
+// (II2) and, for ZNCC, img2 (II1).  launch_window_map fills columns [m0, m1) of
+// `cols`: column m reads integral columns up to m - SM2 + IS2.
+struct WindowMap {
+  float2* ws = nullptr;
+  double* wd = nullptr;
+  double2* wz = nullptr;
+  int ldw = 0, cols = 0;
+  size_t bytes = 0;
+};
+WindowMap window_map(int H, int W, int IS1, int IS2, int SM1, int SM2, int alg, bool SN, void* base);
+cudaError_t launch_window_map(const double* II2, const double* II1, int H, int W, int IS1, int IS2, int SM1, int SM2,
+                              const WindowMap& m, int m0, int m1, cudaStream_t s);
 // passes whose kernel takes the map
-bool piv2d_takes_map(int IS1, int IS2, int SM1, int SM2, int alg, bool SN);
+bool piv2d_takes_map(int IS1, int IS2, int SM1, int SM2, int alg, bool SN, bool pred);
 
 // The same for a column-major H x W x D volume: out is (H+1) x (W+1) x (D+1),
 // first plane zero; scratch holds integral3d_scratch_bytes(H, W, D) bytes.

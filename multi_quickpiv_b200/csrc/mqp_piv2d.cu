@@ -105,10 +105,11 @@ cudaError_t launch_piv2d_batch(const Piv2dBatch& b, cudaStream_t s, std::string&
   return cudaErrorInvalidValue;
 }
 
-bool piv2d_takes_map(int IS1, int IS2, int SM1, int SM2, int alg, bool SN) {
-  (void)SN;
-  return alg == ALG_NSQECC && !direct2d_ok(IS1, IS2, SM1, SM2) && piv2d_fft_len(IS1 + 2 * SM1, IS2 + 2 * SM2) == 64 &&
-         IS1 <= 32 && IS2 <= 32;
+bool piv2d_takes_map(int IS1, int IS2, int SM1, int SM2, int alg, bool SN, bool pred) {
+  if (direct2d_ok(IS1, IS2, SM1, SM2) || piv2d_local_sums(IS1, IS2, SM1, SM2, alg)) return false;
+  // SN: only the strip kernel reads the map then
+  if (SN) return alg == ALG_NSQECC && !pred && IS1 <= 32 && IS2 <= 32 && piv2d_fft_len(IS1 + 2 * SM1, IS2 + 2 * SM2) == 64;
+  return alg == ALG_NSQECC || alg == ALG_ZNCC;
 }
 
 cudaError_t launch_piv2d(const Piv2dArgs& a, int alg, cudaStream_t s, std::string& err) {

@@ -60,6 +60,7 @@ struct Piv2dArgs {
   float2* huge;          // FFT length 256 (mqp_piv2d_huge.cuh): one scratch slot per resident block
   const float2* ws;      // window-sum map of img2^2 (mqp_finish.cuh), or null: read the integral image
   const double* wd;      // SN passes: the map's sums in FP64
+  const double2* wz;     // ZNCC: map of the sums of img2^2 and img2, or null
   int ldw;               // their column length
 };
 

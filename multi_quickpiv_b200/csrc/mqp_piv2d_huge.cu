@@ -7,6 +7,7 @@
 
 #include <string>
 
+#include "mqp_finish.cuh"
 #include "mqp_internal.h"
 #include "mqp_piv2d_huge.cuh"
 
@@ -134,6 +135,20 @@ __device__ __forceinline__ void huge_ia(const Piv2dArgs& a, long long ia, float2
   R.hi2 = 2 * a.SM2 - g.brb2;
   R.shi1 = 2 * a.SM1 - 1 - g.brb1;
   R.shi2 = 2 * a.SM2 - 1 - g.brb2;
+  if (finish_fast(a)) {
+    auto at = [&](int s1, int s2) { return cc[s1 + P1 * s2]; };
+    const int bidx = finish_search<ALG, HUGE_THREADS, 0>(a, g, sc, R, t, P1, 1.0, at, nullptr, red);
+    if (warp == 0) {
+      double r1 = -1.0, r2 = -1.0;  // no peak: 1-based (0, 0), displacement -(SM+1)
+      if (bidx >= 0) finish_refine<ALG, 0>(a, g, sc, bidx % P1, bidx / P1, lane, 1.0, at, nullptr, r1, r2);
+      if (lane == 0) {
+        a.VF[2 * vfo + 0] = r1 - a.SM1 + d1;
+        a.VF[2 * vfo + 1] = r2 - a.SM2 + d2;
+      }
+    }
+    __syncthreads();  // the reduction slots and the scratch slot are reused by the next IA
+    return;
+  }
   PeakAcc acc;
   acc.best = 0.0;
   acc.bidx = -1;

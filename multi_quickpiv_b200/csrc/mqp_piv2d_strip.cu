@@ -24,9 +24,9 @@
 // Bound by instruction issue and supply: 9.5k warp instructions per IA (15.3k
 // before), issue active 45 %, stalls led by no_instruction (1.25 warps per
 // issue) and the barrier after the rows (1.07).  Measured on B200 (kernel,
-// one warp per IA -> strips): 2048^2 NSQECC step 8 2113 -> 1365 us, FFTCC 1270 ->
-// 1155; 1024x1280 NSQECC step 16 199 -> 113; 2048^2 NSQECC step 16 with SN 589 ->
-// 446; 256^2 FFTCC Float64 step 16 35 -> 23.
+// one warp per IA -> strips): 2048^2 NSQECC step 8 2113 -> 1403 us, FFTCC 1270 ->
+// 1197; 1024x1280 NSQECC step 16 199 -> 106; 2048^2 NSQECC step 16 with SN 589 ->
+// 432; 256^2 FFTCC Float64 step 16 35 -> 23.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -44,7 +44,8 @@ namespace {
 constexpr int SN_ = 64;            // FFT length
 constexpr int SM_ = SN_ / 2;       // spectrum columns per IA: one per lane
 // Four warps, three blocks to an SM (168 registers): twelve warps.  Measured on
-// the 2048^2 NSQECC pass at step 8: 1365 us so, 1592 with two blocks (255
+// the 2048^2 NSQECC pass at step 8: 1403 us so, 1775 with four (128 registers,
+// 1.5 KB of spill), 1592 with two (255
 // registers, no spill), 1653 with one block of eight warps and IAs; block
 // sizes that are not a multiple of four warps load the SM's quarters unevenly.
 constexpr int STRIP_WARPS = 4, STRIP_BLOCKS = 3;
@@ -224,6 +225,123 @@ __device__ __forceinline__ void strip_product(int lane, int h, uint32_t tm, floa
   if (lane == 0) {
 #pragma unroll
     for (int m = 0; m < M; ++m) t[m] = pk[2 * M + m];
+  }
+}
+
+// Peak (first_fullovp_peak), SN and Gaussian fit of one IA from its plane (rows
+// below 32) and tail rows.  Not inlined: the transforms before it have the
+// registers to themselves.
+template <int ALG, bool SN>
+__device__ __noinline__ void strip_finish(const Piv2dArgs& a, int v1, int v2, double sumF2, const float* plane,
+                                          const float* tailp, int lane) {
+  const int P1 = 2 * a.SM1 + 1, P2 = 2 * a.SM2 + 1, lane_rows = P1 < 32 ? P1 : 32;
+  const IAGeom g = ia_geom(a, v1, v2);
+  const long long vfo = (long long)v1 + (long long)a.vf1 * v2;
+  IAScalars sc;
+  sc.meanF = sc.meanG = 0.0;
+  sc.sumF2 = sumF2;
+  const double scale = cc_scale<SN_>();
+  auto cc = [&](int s1, int s2) {
+    return s1 < lane_rows ? plane[s1 * P2 + s2] : tailp[(s1 - lane_rows) * P2 + s2];
+  };
+  LagRanges R;
+  R.lo1 = g.tlf1;
+  R.hi1 = 2 * a.SM1 - g.brb1;
+  R.lo2 = g.tlf2;
+  R.hi2 = 2 * a.SM2 - g.brb2;
+  R.shi1 = 2 * a.SM1 - 1 - g.brb1;
+  R.shi2 = 2 * a.SM2 - 1 - g.brb2;
+  int bidx = -1;
+  double sn = 0.0;
+  if (SN) {
+    // the similarities are FP32 values (FFTCC: before the transforms' scale),
+    // so peak and maximum compare in FP32; only the sum is FP64
+    float best = 0.f, smax = -INFINITY;
+    double ssum = 0.0;
+    auto take = [&](int s1, int s2, float v) {
+      if (v > best || (v == best && s1 + P1 * s2 < bidx)) {
+        best = v;
+        bidx = s1 + P1 * s2;
+      }
+      if (s1 <= R.shi1 && s2 <= R.shi2) {
+        smax = (v > smax || v != v) ? v : smax;
+        ssum += ALG == ALG_FFTCC ? (double)v * scale : (double)v;
+      }
+    };
+    if (ALG == ALG_FFTCC) {
+      if (lane < lane_rows && lane >= R.lo1 && lane <= R.hi1)
+        for (int s2 = R.lo2; s2 <= R.hi2; ++s2) take(lane, s2, cc(lane, s2));
+      for (int s1 = lane_rows > R.lo1 ? lane_rows : R.lo1; s1 <= R.hi1; ++s1)
+        for (int s2 = R.lo2 + lane; s2 <= R.hi2; s2 += 32) take(s1, s2, cc(s1, s2));
+    } else if (a.wd) {
+      const int e1 = min(lag_mapped_max(a.SM1, a.IS1, g.g01, g.hi1, a.H), R.hi1);
+      const int e2 = min(lag_mapped_max(a.SM2, a.IS2, g.g02, g.hi2, a.W), R.hi2);
+      // similarity_value with the square root and the FP64 sum of the map
+      const float sqF = sqrtf((float)sc.sumF2);
+      const long long w0 = (g.g01 + a.SM1) + (long long)a.ldw * (g.g02 + a.SM2);
+      auto sim = [&](float q, double S2, float c) {
+        const float d = q * sqF;
+        const double n = (sc.sumF2 - 2.0 * ((double)c * scale)) + S2;
+        return d / (float)(n + (double)d);
+      };
+      constexpr int B = 8;  // lags whose sums are loaded before any is used
+      if (lane < lane_rows && lane >= R.lo1 && lane <= e1) {
+        for (int b = R.lo2; b <= e2; b += B) {
+          double S2[B];
+          float q[B];
+#pragma unroll
+          for (int k = 0; k < B; ++k) {  // past the box: the last column again, not taken
+            const long long w = w0 + lane + (long long)a.ldw * min(b + k, e2);
+            S2[k] = __ldg(a.wd + w);
+            q[k] = __ldg(&a.ws[w].y);
+          }
+          mqp_no_hoist();
+#pragma unroll
+          for (int k = 0; k < B; ++k)
+            if (b + k <= e2) take(lane, b + k, sim(q[k], S2[k], cc(lane, b + k)));
+        }
+      }
+      for (int s1 = lane_rows > R.lo1 ? lane_rows : R.lo1; s1 <= e1; ++s1)
+        for (int s2 = R.lo2 + lane; s2 <= e2; s2 += 32) {
+          const long long w = w0 + s1 + (long long)a.ldw * s2;
+          take(s1, s2, sim(__ldg(&a.ws[w].y), __ldg(a.wd + w), cc(s1, s2)));
+        }
+      unmapped_lags(R, e1, e2, lane, [&](int s1, int s2) {
+        take(s1, s2, (float)finish_one<ALG>(a, g, sc, s1, s2, (double)cc(s1, s2) * scale));
+      });
+    } else {
+      const int w2 = R.hi2 - R.lo2 + 1, total = (R.hi1 - R.lo1 + 1) * w2;
+#pragma unroll 1
+      for (int q = lane; q < total; q += 32) {
+        const int s1 = R.lo1 + q / w2, s2 = R.lo2 + q % w2;
+        take(s1, s2, (float)finish_one<ALG>(a, g, sc, s1, s2, (double)cc(s1, s2) * scale));
+      }
+    }
+    // merged as peak_merge: the largest value, of equal ones the lowest index
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      const float ob = __shfl_xor_sync(0xffffffffu, best, off), om = __shfl_xor_sync(0xffffffffu, smax, off);
+      const int oi = __shfl_xor_sync(0xffffffffu, bidx, off);
+      if (oi >= 0 && (bidx < 0 || ob > best || (ob == best && oi < bidx))) {
+        best = ob;
+        bidx = oi;
+      }
+      smax = (om > smax || om != om) ? om : smax;
+    }
+    ssum = sum32(ssum);
+    // compute_SN (src/utils/piv_ops.jl:336-367) over [TLF_off, 2SM-1-BRB_off]
+    const double top = ALG == ALG_FFTCC ? (double)smax * scale : (double)smax;
+    const double len = (double)(R.shi1 - R.lo1 + 1) * (double)(R.shi2 - R.lo2 + 1);
+    sn = top / ((ssum - top) / (len - 1.0));
+  } else {
+    bidx = finish_search<ALG, 32, 0>(a, g, sc, R, lane, P1, scale, cc, nullptr, nullptr);
+  }
+  double r1 = -1.0, r2 = -1.0;  // no peak: 1-based (0, 0), displacement -(SM+1)
+  if (bidx >= 0) finish_refine<ALG, 0>(a, g, sc, bidx % P1, bidx / P1, lane, scale, cc, nullptr, r1, r2);
+  if (lane == 0) {
+    a.VF[2 * vfo + 0] = r1 - a.SM1;
+    a.VF[2 * vfo + 1] = r2 - a.SM2;
+    if (SN) a.SN[vfo] = sn;
   }
 }
 
@@ -423,116 +541,11 @@ __device__ __forceinline__ void strip_ia(const Piv2dArgs& a, const StripCfg& c, 
     if (c.wpi == 2 && role == 0) return;
   }
   __syncwarp();
-
-  // ---- peak (first_fullovp_peak), SN, Gaussian fit ----
-  const float* plane = reinterpret_cast<const float*>(priv);
-  const double scale = cc_scale<N>();
-  auto cc = [&](int s1, int s2) {
-    return s1 < lane_rows ? plane[s1 * P2 + s2] : tailp[(s1 - lane_rows) * P2 + s2];
-  };
-  LagRanges R;
-  R.lo1 = g.tlf1;
-  R.hi1 = 2 * a.SM1 - g.brb1;
-  R.lo2 = g.tlf2;
-  R.hi2 = 2 * a.SM2 - g.brb2;
-  R.shi1 = 2 * a.SM1 - 1 - g.brb1;
-  R.shi2 = 2 * a.SM2 - 1 - g.brb2;
-  int bidx = -1;
-  double sn = 0.0;
-  if (SN) {
-    // the similarities are FP32 values (FFTCC: before the transforms' scale),
-    // so peak and maximum compare in FP32; only the sum is FP64
-    float best = 0.f, smax = -INFINITY;
-    double ssum = 0.0;
-    auto take = [&](int s1, int s2, float v) {
-      if (v > best || (v == best && s1 + P1 * s2 < bidx)) {
-        best = v;
-        bidx = s1 + P1 * s2;
-      }
-      if (s1 <= R.shi1 && s2 <= R.shi2) {
-        smax = (v > smax || v != v) ? v : smax;
-        ssum += ALG == ALG_FFTCC ? (double)v * scale : (double)v;
-      }
-    };
-    if (ALG == ALG_FFTCC) {
-      if (lane < lane_rows && lane >= R.lo1 && lane <= R.hi1)
-        for (int s2 = R.lo2; s2 <= R.hi2; ++s2) take(lane, s2, cc(lane, s2));
-      for (int s1 = lane_rows > R.lo1 ? lane_rows : R.lo1; s1 <= R.hi1; ++s1)
-        for (int s2 = R.lo2 + lane; s2 <= R.hi2; s2 += 32) take(s1, s2, cc(s1, s2));
-    } else if (a.wd) {
-      const int e1 = min(lag_mapped_max(a.SM1, a.IS1, g.g01, g.hi1, a.H), R.hi1);
-      const int e2 = min(lag_mapped_max(a.SM2, a.IS2, g.g02, g.hi2, a.W), R.hi2);
-      // similarity_value with the square root and the FP64 sum of the map
-      const float sqF = sqrtf((float)sc.sumF2);
-      const long long w0 = (g.g01 + a.SM1) + (long long)a.ldw * (g.g02 + a.SM2);
-      auto sim = [&](float q, double S2, float c) {
-        const float d = q * sqF;
-        const double n = (sc.sumF2 - 2.0 * ((double)c * scale)) + S2;
-        return d / (float)(n + (double)d);
-      };
-      constexpr int B = 8;  // lags whose sums are loaded before any is used
-      if (lane < lane_rows && lane >= R.lo1 && lane <= e1) {
-        for (int b = R.lo2; b <= e2; b += B) {
-          double S2[B];
-          float q[B];
-#pragma unroll
-          for (int k = 0; k < B; ++k) {  // past the box: the last column again, not taken
-            const long long w = w0 + lane + (long long)a.ldw * min(b + k, e2);
-            S2[k] = __ldg(a.wd + w);
-            q[k] = __ldg(&a.ws[w].y);
-          }
-          mqp_no_hoist();
-#pragma unroll
-          for (int k = 0; k < B; ++k)
-            if (b + k <= e2) take(lane, b + k, sim(q[k], S2[k], cc(lane, b + k)));
-        }
-      }
-      for (int s1 = lane_rows > R.lo1 ? lane_rows : R.lo1; s1 <= e1; ++s1)
-        for (int s2 = R.lo2 + lane; s2 <= e2; s2 += 32) {
-          const long long w = w0 + s1 + (long long)a.ldw * s2;
-          take(s1, s2, sim(__ldg(&a.ws[w].y), __ldg(a.wd + w), cc(s1, s2)));
-        }
-      unmapped_lags(R, e1, e2, lane, [&](int s1, int s2) {
-        take(s1, s2, (float)finish_one<ALG>(a, g, sc, s1, s2, (double)cc(s1, s2) * scale));
-      });
-    } else {
-      const int w2 = R.hi2 - R.lo2 + 1, total = (R.hi1 - R.lo1 + 1) * w2;
-#pragma unroll 1
-      for (int q = lane; q < total; q += 32) {
-        const int s1 = R.lo1 + q / w2, s2 = R.lo2 + q % w2;
-        take(s1, s2, (float)finish_one<ALG>(a, g, sc, s1, s2, (double)cc(s1, s2) * scale));
-      }
-    }
-    // merged as peak_merge: the largest value, of equal ones the lowest index
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      const float ob = __shfl_xor_sync(0xffffffffu, best, off), om = __shfl_xor_sync(0xffffffffu, smax, off);
-      const int oi = __shfl_xor_sync(0xffffffffu, bidx, off);
-      if (oi >= 0 && (bidx < 0 || ob > best || (ob == best && oi < bidx))) {
-        best = ob;
-        bidx = oi;
-      }
-      smax = (om > smax || om != om) ? om : smax;
-    }
-    ssum = sum32(ssum);
-    // compute_SN (src/utils/piv_ops.jl:336-367) over [TLF_off, 2SM-1-BRB_off]
-    const double top = ALG == ALG_FFTCC ? (double)smax * scale : (double)smax;
-    const double len = (double)(R.shi1 - R.lo1 + 1) * (double)(R.shi2 - R.lo2 + 1);
-    sn = top / ((ssum - top) / (len - 1.0));
-  } else {
-    bidx = finish_search<ALG>(a, g, sc, R, lane, lane_rows, P1, scale, cc);
-  }
-  double r1 = -1.0, r2 = -1.0;  // no peak: 1-based (0, 0), displacement -(SM+1)
-  if (bidx >= 0) finish_refine<ALG>(a, g, sc, bidx % P1, bidx / P1, lane, scale, cc, r1, r2);
-  if (lane == 0) {
-    a.VF[2 * vfo + 0] = r1 - a.SM1;
-    a.VF[2 * vfo + 1] = r2 - a.SM2;
-    if (SN) a.SN[vfo] = sn;
-  }
+  strip_finish<ALG, SN>(a, v1, v2, sc.sumF2, reinterpret_cast<const float*>(priv), tailp, lane);
 }
 
 template <int ALG, typename T, bool SN>
-__global__ void __launch_bounds__(STRIP_WARPS * 32, STRIP_BLOCKS) strip_kernel(Piv2dArgs a, StripCfg c) {
+__global__ void __launch_bounds__(STRIP_WARPS * 32, STRIP_BLOCKS) strip_kernel(const __grid_constant__ Piv2dArgs a, StripCfg c) {
   extern __shared__ __align__(16) float2 smem[];
   constexpr int N = SN_;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -622,7 +635,6 @@ cudaError_t strip_dt(const Piv2dArgs& a, const StripCfg& c, cudaStream_t s, std:
 bool piv2d_strip_ok(const Piv2dArgs& a, int alg) {
   if (alg != ALG_FFTCC && alg != ALG_NSQECC) return false;
   if (a.pred || a.planes) return false;
-  if (alg == ALG_NSQECC && !a.SN && !a.ws) return false;
   if (a.IS1 > SM_ || a.IS2 > SM_ || a.vf1 < 1 || a.st1 > a.IS1) return false;
   if (piv2d_fft_len(a.IS1 + 2 * a.SM1, a.IS2 + 2 * a.SM2) != SN_) return false;
   if (2 * a.SM1 + 1 > 36) return false;  // one lag row per lane, up to four by direct sums

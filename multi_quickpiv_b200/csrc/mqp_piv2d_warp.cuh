@@ -11,6 +11,7 @@
 
 #include <string>
 
+#include "mqp_finish.cuh"
 #include "mqp_internal.h"
 #include "mqp_stage.cuh"
 
@@ -281,6 +282,23 @@ __device__ __forceinline__ void piv2d_ia(const Piv2dArgs& a, long long ia, float
   R.hi2 = 2 * a.SM2 - g.brb2;
   R.shi1 = 2 * a.SM1 - 1 - g.brb1;
   R.shi2 = 2 * a.SM2 - 1 - g.brb2;
+  if constexpr (!MASKED) {
+    if (finish_fast(a)) {
+      auto cc = [&](int s1, int s2) { return (float)plane[s1 * P2 + s2]; };  // exact: FP32 times a power of two
+      const int bidx = finish_search<ALG, 32, LW ? N : 0>(a, g, sc, R, lane, P1, 1.0, cc, lw, nullptr);
+      double r1 = -1.0, r2 = -1.0;  // no peak: 1-based (0, 0), displacement -(SM+1)
+      if (bidx >= 0)
+        finish_refine<ALG, LW ? N : 0>(a, g, sc, bidx % P1, bidx / P1, lane, 1.0, cc, lw, r1, r2);
+      __syncwarp();
+      if (LW) stage_next();
+      if (lane == 0) {
+        a.VF[2 * vfo + 0] = r1 - a.SM1 + d1;
+        a.VF[2 * vfo + 1] = r2 - a.SM2 + d2;
+      }
+      __syncwarp();
+      return;
+    }
+  }
   PeakAcc acc;
   acc.best = 0.0;
   acc.bidx = -1;
