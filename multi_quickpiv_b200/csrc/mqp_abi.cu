@@ -272,21 +272,45 @@ int run_pass_3d(mqp_ctx* ctx, const Problem& pb, const mqp_params* p, const void
     }
   }
   const bool direct = mqp::direct3d_ok(pb.IS, pb.SM);  // small windows: spatial correlation, no chunk scratch
-  // chunk scratch: Gz | Fz | C | C2 | V | state | K3a parts | K3c parts
-  const size_t per_ia = mqp::piv3d_scratch_bytes_per_ia(pb.IS, pb.SM, pb.alg);
+  // chunk scratch: Gz | Fz | C | C2 | V | state | K3a parts | K3c parts; with
+  // z-spectra shared per layer, those first and no Gz / Fz.  Sharing pays where
+  // the layer's windows hold more lines than the two images, and its planes
+  // take at most half of the scratch budget.
   const int64_t n = ia_end - ia_begin;
-  int64_t chunk = ctx->chunk3d > 0 ? ctx->chunk3d : (int64_t)(ctx->chunk3d_budget / per_ia);
+  const double lines = (double)(pb.vf[0] * pb.vf[1]) * ((double)SS[0] * SS[1] + (double)pb.IS[0] * pb.IS[1]);
+  size_t shared_b = 0;
+  if (!direct && !dpred && (pb.alg == mqp::ALG_FFTCC || pb.alg == mqp::ALG_NSQECC) && W <= 65535 &&
+      lines > 2.0 * (double)H * (double)W) {
+    shared_b = align256(mqp::piv3d_shared_bytes(pb.IS, pb.SM, H, W));
+    if (shared_b > ctx->chunk3d_budget / 2) shared_b = 0;
+  }
+  const bool shared = shared_b != 0;
+  const size_t per_ia = mqp::piv3d_scratch_bytes_per_ia(pb.IS, pb.SM, pb.alg, shared);
+  const int64_t layer = pb.vf[0] * pb.vf[1];
+  int64_t chunk, layers = 0;
+  if (ctx->chunk3d > 0) {
+    chunk = ctx->chunk3d;
+  } else if (shared && shared_b + per_ia * (size_t)layer <= ctx->chunk3d_budget) {  // whole layers
+    chunk = layer * (int64_t)(ctx->chunk3d_budget / (shared_b + per_ia * (size_t)layer));
+  } else {
+    chunk = (int64_t)((ctx->chunk3d_budget - shared_b) / per_ia);
+  }
   if (chunk < 1) chunk = 1;
   if (chunk > 65535) chunk = 65535;
   if (chunk > n) chunk = n;
+  if (shared) layers = std::min<int64_t>(std::max<int64_t>(1, ctx->chunk3d_budget / 2 / shared_b), (chunk + layer - 1) / layer);
   for (int d = 0; d < 3; ++d) {
     a.IS[d] = pb.IS[d];
     a.SM[d] = pb.SM[d];
   }
+  a.H = H;
+  a.W = W;
   if (!direct) {
-    if ((e = ctx->scratch3d.ensure(mqp::piv3d_scratch_bytes(pb.IS, pb.SM, pb.alg, chunk))) != cudaSuccess)
+    const size_t sb = shared_b * (size_t)layers;
+    if ((e = ctx->scratch3d.ensure(sb + mqp::piv3d_scratch_bytes(pb.IS, pb.SM, pb.alg, chunk, shared))) != cudaSuccess)
       return cuda_fail(ctx, e, "3D scratch");
-    mqp::piv3d_bind_scratch(a, pb.alg, chunk, (char*)ctx->scratch3d.ptr);
+    if (shared) mqp::piv3d_bind_shared(a, (int)layers, (char*)ctx->scratch3d.ptr);
+    mqp::piv3d_bind_scratch(a, pb.alg, chunk, (char*)ctx->scratch3d.ptr + sb, shared);
   }
   a.img1 = d1;
   a.img2 = d2;
@@ -311,6 +335,17 @@ int run_pass_3d(mqp_ctx* ctx, const Problem& pb, const mqp_params* p, const void
   a.ia_end = ia_end;
   a.threshold = p->threshold;
   a.mask_threshold = p->mask_threshold;
+  if (!direct && need_g2 && !dSN && !dplanes) {
+    // window-sum map; without memory for it the kernels read the integral volumes
+    e = ctx->wmap.ensure(mqp::window_map3_bytes(a, pb.alg));
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+    } else {
+      ProfileScope ps(ctx, s, 0, 0);
+      if (e != cudaSuccess || (e = mqp::launch_window_map3(a, pb.alg, ctx->wmap.ptr, s)) != cudaSuccess)
+        return cuda_fail(ctx, e, "window-sum map");
+    }
+  }
   std::string err;
   {
     ProfileScope ps(ctx, s, 1, ia_end - ia_begin);

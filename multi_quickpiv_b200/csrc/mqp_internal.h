@@ -138,12 +138,22 @@ cudaError_t launch_piv2d_big_batch(const Piv2dBatch& b, cudaStream_t s, std::str
 // a.ia_end) in chunks of `chunk` IAs (the scratch pointers of `a` must hold
 // chunk IAs).
 int piv3d_fft_len(const int SS[3]);
-size_t piv3d_scratch_bytes_per_ia(const int IS[3], const int SM[3], int alg);
+size_t piv3d_scratch_bytes_per_ia(const int IS[3], const int SM[3], int alg, bool shared = false);
 // chunk scratch of the 3D kernels for `chunk` IAs, and Piv3dArgs' scratch
 // pointers bound into it (a.IS / a.SM set)
-size_t piv3d_scratch_bytes(const int IS[3], const int SM[3], int alg, long long chunk);
-void piv3d_bind_scratch(Piv3dArgs& a, int alg, long long chunk, char* base);
+size_t piv3d_scratch_bytes(const int IS[3], const int SM[3], int alg, long long chunk, bool shared = false);
+void piv3d_bind_scratch(Piv3dArgs& a, int alg, long long chunk, char* base, bool shared = false);
 cudaError_t launch_piv3d(const Piv3dArgs& a, int alg, long long chunk, cudaStream_t s, std::string& err);
+// FFTCC and NSQECC passes without a predictor may share a layer's z-spectra
+// between its IAs: scratch bytes per layer, and Piv3dArgs' pointers into room
+// for `layers` of them (a.IS / a.SM / a.H / a.W set).  Their chunk scratch holds no
+// Gz / Fz then.
+size_t piv3d_shared_bytes(const int IS[3], const int SM[3], long long H, long long W);
+void piv3d_bind_shared(Piv3dArgs& a, int layers, char* base);
+// Window-sum map of an NSQECC or ZNCC pass without SN (geometry and integral
+// volumes set in `a`): bytes, and the kernel, which binds a.ws / a.wz to `base`.
+size_t window_map3_bytes(const Piv3dArgs& a, int alg);
+cudaError_t launch_window_map3(Piv3dArgs& a, int alg, void* base, cudaStream_t s);
 
 // Multi-pass refinement: the fine pass's predictor from the coarse vectors.
 cudaError_t launch_predictor(const PredArgs& a, cudaStream_t s);

@@ -5,8 +5,10 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <string>
 
+#include "mqp_finish3.cuh"
 #include "mqp_internal.h"
 
 namespace mqp {
@@ -97,8 +99,98 @@ __global__ void k3a_merge_kernel(Piv3dArgs a, long long n) {
   a.state[ci] = s;
 }
 
+// z-spectra of whole image layers: without a predictor every IA of one
+// vector-field z index reads the same z window, so a line's r2c along dim 3
+// (k3a_line) serves every IA that covers it (16 at step 16 and windows of 64).
+// Thread per line; blockIdx.z = 2 layer + (0: G, 1: F).  FFTCC and NSQECC (ZNCC
+// subtracts each IA's own mean first).
+template <int N, bool FPRUNE, typename T>
+__global__ void __launch_bounds__(256) k3s_lines_kernel(Piv3dArgs a) {
+  constexpr int M = N / 2;
+  const long long HW = (long long)a.H * a.W;
+  const int x1 = blockIdx.x * blockDim.x + threadIdx.x, x2 = blockIdx.y, l = blockIdx.z >> 1;
+  if (x1 >= a.H) return;
+  const IAGeom3 g = ia_geom3(a, (long long)a.vf[0] * a.vf[1] * (a.l0 + l));
+  const long long at = x1 + (long long)a.H * x2;
+  float2* out = ((blockIdx.z & 1) ? a.Fs : a.Gs) + (x1 + a.pitch * x2 + a.lstride * l);
+  float2 z[M];
+  if (blockIdx.z & 1) {
+    const T* p = reinterpret_cast<const T*>(a.img1) + (at + HW * g.ir[2]);
+    constexpr int FLIM = Lay3<N, FPRUNE>::NF;
+#pragma unroll
+    for (int n = 0; n < M; ++n) {
+      const int u = 2 * n, v = 2 * n + 1;
+      z[n] = make_float2(u < FLIM && u < a.IS[2] ? (float)ldg_px<T>(p, HW * u) : 0.f,
+                         v < FLIM && v < a.IS[2] ? (float)ldg_px<T>(p, HW * v) : 0.f);
+    }
+    r2c_line_store<N, FPRUNE ? M / 2 : M>(z, out, a.zplane);
+  } else {
+    const T* p = reinterpret_cast<const T*>(a.img2) + (at + HW * g.g0[2]);
+    const int zl = g.lo[2], zh = g.hi[2];
+#pragma unroll
+    for (int n = 0; n < M; ++n) {
+      const int u = 2 * n, v = 2 * n + 1;
+      z[n] = make_float2(u >= zl && u < zh ? (float)ldg_px<T>(p, HW * u) : 0.f,
+                         v >= zl && v < zh ? (float)ldg_px<T>(p, HW * v) : 0.f);
+    }
+    r2c_line_store<N, M>(z, out, a.zplane);
+  }
+}
+
+// With shared z-spectra: an IA's skip maximum and sumF2, a block per IA.
+template <typename T, int ALG>
+__global__ void __launch_bounds__(K3A_THREADS) k3s_state_kernel(Piv3dArgs a) {
+  const long long ci = blockIdx.x;
+  const IAGeom3 g = ia_geom3(a, a.ia_begin + ci);
+  const long long HW = (long long)a.H * a.W;
+  double vmax = -INFINITY, sumsq = 0.0;
+  const int nl = a.IS[0] * a.IS[1];
+  constexpr int LB = 4;  // lines a thread sums at once: as many independent chains
+  for (int l0 = threadIdx.x; l0 < nl; l0 += LB * K3A_THREADS) {
+    const T* p[LB];
+    bool in[LB];
+    double sq[LB];
+#pragma unroll
+    for (int k = 0; k < LB; ++k) {
+      const int line = l0 + k * K3A_THREADS;
+      in[k] = line < nl;
+      const int x1 = in[k] ? line % a.IS[0] : 0, x2 = in[k] ? line / a.IS[0] : 0;
+      p[k] = reinterpret_cast<const T*>(a.img1) +
+             ((long long)(g.ir[0] + x1) + (long long)a.H * ((long long)(g.ir[1] + x2) + (long long)a.W * g.ir[2]));
+      sq[k] = 0.0;
+    }
+#pragma unroll 4
+    for (int x = 0; x < a.IS[2]; ++x) {
+#pragma unroll
+      for (int k = 0; k < LB; ++k) {
+        const double r = (double)ldg_px<T>(p[k], HW * x);
+        vmax = in[k] && r > vmax ? r : vmax;
+        sq[k] += r * r;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < LB; ++k) sumsq += in[k] ? sq[k] : 0.0;
+  }
+  __shared__ double red[2][K3A_THREADS / 32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  vmax = warp_max3(vmax);
+  sumsq = warp_sum3(sumsq);
+  if (lane == 0) {
+    red[0][warp] = vmax;
+    red[1][warp] = sumsq;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < K3A_THREADS / 32; ++w) {
+      vmax = fmax(vmax, red[0][w]);
+      sumsq += red[1][w];
+    }
+    a.state[ci] = IA3State{sumsq, 0.0, 0.0, skip_test3(a, ALG, vmax, vmax) ? 1 : 0, 0};
+  }
+}
+
 // One block of 2N threads (a pair per line) per (k3, IA) slab.
-template <int N, bool FPRUNE>
+template <int N, bool FPRUNE, bool SHARED>
 __global__ void __launch_bounds__(2 * N) k3b_kernel(Piv3dArgs a, float2* C) {
   using L = Lay3<N, FPRUNE>;
   constexpr int M = N / 2;
@@ -111,7 +203,8 @@ __global__ void __launch_bounds__(2 * N) k3b_kernel(Piv3dArgs a, float2* C) {
   float2* S = sm;
   float2* SF = sm + N * L::SSTR;
   const int t = threadIdx.x % N, h = threadIdx.x / N;
-  k3b_rows<N, FPRUNE>(a, g, ci, k3, t, h, S, SF);
+  if (SHARED) k3b_rows_shared<N, FPRUNE>(a, g, k3, t, h, S, SF);
+  else k3b_rows<N, FPRUNE>(a, g, ci, k3, t, h, S, SF);
   __syncthreads();
   {
     float2 y[M];
@@ -232,35 +325,302 @@ __global__ void k3c_merge_kernel(Piv3dArgs a, long long n, int parts) {
   k3c_final(a, g, ci, lag_ranges3(a, g), b, bi, mx, sum);
 }
 
+// K3c of a pass that ends in the walk (finish3_fast): the lag pair's inverse
+// along k3, the raw correlations to V (the fit's neighbourhood), FP32
+// approximations of the similarity to the block's two largest.  With the
+// window sums in one 8-byte read per lag (ZNCC: 16) instead of eight FP64 ones
+// (sixteen), no FP64 square roots, quotients or compares and 128 registers
+// instead of 224..237, two blocks run on an SM.
+template <int N, int ALG>
+__global__ void __launch_bounds__(K3C_THREADS, N <= 64 ? 2 : 1) k3c_walk_kernel(Piv3dArgs a) {
+  constexpr int M = N / 2, K3 = M + 1;
+  const int part = blockIdx.x, parts = gridDim.x;
+  const long long ci = blockIdx.y;
+  const int P1 = 2 * a.SM[0] + 1, P2 = 2 * a.SM[1] + 1, P3 = 2 * a.SM[2] + 1, P12 = P1 * P2;
+  const int q0 = P12 * part / parts, q1 = P12 * (part + 1) / parts;
+  const IA3State st = a.state[ci];
+  if (st.skip) return;
+  const IAGeom3 g = ia_geom3(a, a.ia_begin + ci);
+  const LagRanges3 R = lag_ranges3(a, g);
+  const float sqF = sqrtf((float)st.sumF2), F2 = (float)st.sumF2;
+  const float fscale = (float)cc_scale3<N>(), m2 = -2.f * fscale;
+  const bool map = ALG == ALG_NSQECC ? a.ws != nullptr : (ALG == ALG_ZNCC && a.wz != nullptr);
+  int e[3];  // last lags whose sums the map holds (without a map: none)
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const int size = d == 0 ? a.H : (d == 1 ? a.W : a.D);
+    e[d] = map ? min(R.hi[d], lag_mapped_max(a.SM[d], a.IS[d], g.g0[d], g.hi[d], size)) : R.lo[d] - 1;
+  }
+  TopTwo t;
+  t.b1 = t.b2 = 0.f;
+  t.idx = -1;
+#pragma unroll 1
+  for (int q = q0 + threadIdx.x; q < q1; q += blockDim.x) {
+    const int s1 = q % P1, s2 = q / P1;
+    float2 x[M];
+    c2r_k3<N>(a.C + ci * K3 * P12 + q, P12, x);
+    float* vdst = a.V + ci * P12 * P3 + q;
+    const bool in = s1 >= R.lo[0] && s1 <= (ALG == ALG_FFTCC ? R.hi[0] : e[0]) && s2 >= R.lo[1] &&
+                    s2 <= (ALG == ALG_FFTCC ? R.hi[1] : e[1]);
+    const int last = ALG == ALG_FFTCC ? R.hi[2] : e[2];
+    const long long w0 = (g.g0[0] + s1 + a.SM[0]) +
+                         (long long)a.ldw1 * ((g.g0[1] + s2 + a.SM[1]) + (long long)a.ldw2 * (g.g0[2] + a.SM[2]));
+    const long long wk = (long long)a.ldw1 * a.ldw2;
+    double nrc = 0.0;
+    if (ALG == ALG_ZNCC) {
+      int r0, r1, c0, c1;
+      lag_window(s1, a.IS[0], g.g0[0], g.lo[0], g.hi[0], r0, r1);
+      lag_window(s2, a.IS[1], g.g0[1], g.lo[1], g.hi[1], c0, c1);
+      nrc = (double)(r1 - r0) * (double)(c1 - c0);
+    }
+    constexpr int B = ALG == ALG_ZNCC ? 4 : 8;  // lags whose sums are read before any is used
+#pragma unroll
+    for (int b = 0; b < N; b += B) {
+      if (b >= P3) continue;
+      float2 m[B];
+      double2 mz[B];
+      if (ALG != ALG_FFTCC && in && last >= R.lo[2]) {
+#pragma unroll
+        for (int k = 0; k < B; ++k) {
+          const long long w = w0 + wk * min(max(b + k, R.lo[2]), last);
+          if (ALG == ALG_NSQECC) m[k] = __ldg(a.ws + w);
+          else mz[k] = __ldg(a.wz + w);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < B; ++k) {
+        const int s3 = b + k;
+        if (s3 < P3) {
+          const float2 z = x[fpos<M>(s3 >> 1)];
+          const float c = (s3 & 1) ? z.y : z.x;
+          vdst[(long long)s3 * P12] = c;
+          if (in && s3 >= R.lo[2] && s3 <= last) {
+            const int idx = q + P12 * s3;
+            if (ALG == ALG_FFTCC) {
+              first_take(t, c, idx);
+            } else if (ALG == ALG_NSQECC) {
+              const float d = m[k].y * sqF;
+              top_take(t, d * rcp_approx(fmaf(m2, c, F2 + m[k].x) + d), idx);
+            } else {
+              int z0, z1;
+              lag_window(s3, a.IS[2], g.g0[2], g.lo[2], g.hi[2], z0, z1);
+              const double n = nrc * (double)(z1 - z0);
+              const double SG = mz[k].x - 2.0 * st.meanG * mz[k].y + n * st.meanG * st.meanG;
+              top_take(t, c * fscale * rsqrtf((float)(SG > 0.0 ? SG : 0.0)), idx);
+            }
+          }
+        }
+      }
+    }
+  }
+  // lags whose sums the map does not hold, in full
+  if (ALG != ALG_FFTCC && (e[0] < R.hi[0] || e[1] < R.hi[1] || e[2] < R.hi[2])) {
+    __syncthreads();  // V of this part
+#pragma unroll 1
+    for (int q = q0 + threadIdx.x; q < q1; q += blockDim.x) {
+      const int s1 = q % P1, s2 = q / P1;
+      if (s1 < R.lo[0] || s1 > R.hi[0] || s2 < R.lo[1] || s2 > R.hi[1]) continue;
+#pragma unroll 1
+      for (int s3 = s1 <= e[0] && s2 <= e[1] ? max(e[2] + 1, R.lo[2]) : R.lo[2]; s3 <= R.hi[2]; ++s3) {
+        const int idx = q + P12 * s3;
+        const float v = (float)full_sim3<ALG>(a, g, st, s1, s2, s3, (double)a.V[ci * P12 * P3 + idx] * cc_scale3<N>());
+        top_take(t, ALG == ALG_ZNCC ? v * sqF : v, idx);  // on the walk's scale
+      }
+    }
+  }
+  // the block's two largest
+  __shared__ TopPart3 red[K3C_THREADS / 32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    const float o1 = __shfl_xor_sync(0xffffffffu, t.b1, off), o2 = __shfl_xor_sync(0xffffffffu, t.b2, off);
+    const int oi = __shfl_xor_sync(0xffffffffu, t.idx, off);
+    top_merge(t, o1, o2, oi);
+  }
+  if (lane == 0) red[warp] = TopPart3{t.b1, t.b2, t.idx, 0};
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) top_merge(t, red[w].b1, red[w].b2, red[w].idx);
+    reinterpret_cast<TopPart3*>(a.cpart)[ci * parts + part] = TopPart3{t.b1, t.b2, t.idx, 0};
+  }
+}
+
+// A block per IA: the walk's parts, every lag in full where they leave more
+// than one open, and the Gaussian fit with a lane per neighbour.
+constexpr int K3F_THREADS = 128;
+template <int N, int ALG>
+__global__ void __launch_bounds__(K3F_THREADS) k3c_walk_merge_kernel(Piv3dArgs a, int parts) {
+  const long long ci = blockIdx.x, ia = a.ia_begin + ci;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const IA3State st = a.state[ci];
+  if (st.skip) {
+    if (tid == 0) k3c_skipped(a, ci);
+    return;
+  }
+  const IAGeom3 g = ia_geom3(a, ia);
+  const LagRanges3 R = lag_ranges3(a, g);
+  const int P1 = 2 * a.SM[0] + 1, P2 = 2 * a.SM[1] + 1, P3 = 2 * a.SM[2] + 1, P12 = P1 * P2;
+  const float* V = a.V + ci * P12 * P3;
+  const double scale = cc_scale3<N>();
+  const TopPart3* p = reinterpret_cast<const TopPart3*>(a.cpart) + ci * parts;
+  TopTwo t;
+  t.b1 = p[0].b1;
+  t.b2 = p[0].b2;
+  t.idx = p[0].idx;
+  for (int k = 1; k < parts; ++k) top_merge(t, p[k].b1, p[k].b2, p[k].idx);
+  int bidx = t.b1 > 0.f ? t.idx : -1;
+  // an all-zero window has no value above 0; sums outside the normal FP32
+  // range and near ties take the full search
+  const bool zero = ALG != ALG_FFTCC && st.sumF2 == 0.0;
+  const bool full = ALG != ALG_FFTCC && !zero &&
+                    (!(st.sumF2 > 1e-30 && st.sumF2 < 1e30) || (t.b1 > 0.f && t.b2 >= t.b1 * (1.f - PEAK_GAP)));
+  if (zero) bidx = -1;
+  if (full) {
+    double best = 0.0;
+    bidx = -1;
+    const int n1 = R.hi[0] - R.lo[0] + 1, n2 = R.hi[1] - R.lo[1] + 1, n3 = R.hi[2] - R.lo[2] + 1;
+    const int total = n1 > 0 && n2 > 0 && n3 > 0 ? n1 * n2 * n3 : 0;
+    for (int q = tid; q < total; q += K3F_THREADS) {
+      const int s1 = R.lo[0] + q % n1, s2 = R.lo[1] + (q / n1) % n2, s3 = R.lo[2] + q / (n1 * n2);
+      const int idx = s1 + P1 * s2 + P12 * s3;
+      peak_take(full_sim3<ALG>(a, g, st, s1, s2, s3, (double)V[idx] * scale), idx, best, bidx);
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      const double ob = __shfl_xor_sync(0xffffffffu, best, off);
+      const int oi = __shfl_xor_sync(0xffffffffu, bidx, off);
+      peak_merge(best, bidx, ob, oi);
+    }
+    __shared__ double rb[K3F_THREADS / 32];
+    __shared__ int ri[K3F_THREADS / 32];
+    if (lane == 0) {
+      rb[warp] = best;
+      ri[warp] = bidx;
+    }
+    __syncthreads();
+    best = rb[0];
+    bidx = ri[0];
+    for (int w = 1; w < K3F_THREADS / 32; ++w) peak_merge(best, bidx, rb[w], ri[w]);
+  }
+  if (warp != 0) return;
+  double r[3] = {-1.0, -1.0, -1.0};  // no peak: 1-based (0, 0, 0), displacement -(SM+1)
+  if (bidx >= 0) {
+    const int pk[3] = {bidx % P1, (bidx / P1) % P2, bidx / P12};
+    bool inside = true;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      r[d] = pk[d];
+      inside = inside && (pk[d] + 1 > 1 + g.tlf[d]) && (pk[d] + 1 < 1 + 2 * a.SM[d] - g.brb[d]);
+    }
+    if (inside) {
+      // lane = (i + 1) + 3 (j + 1) + 9 (k + 1); the similarity volume is FP32
+      float v = 0.f;
+      if (lane < 27) {
+        const int s1 = pk[0] - 1 + lane % 3, s2 = pk[1] - 1 + (lane / 3) % 3, s3 = pk[2] - 1 + lane / 9;
+        v = (float)full_sim3<ALG>(a, g, st, s1, s2, s3, (double)V[s1 + P1 * s2 + P12 * s3] * scale);
+      }
+      double mn = (double)__shfl_sync(0xffffffffu, v, 0);
+#pragma unroll
+      for (int k = 0; k < 27; ++k) mn = nmin(mn, (double)__shfl_sync(0xffffffffu, v, k));
+      const double lg = lane < 27 ? log(1.0 + (double)v - mn) : 0.0;
+      const int from[7] = {13, 12, 14, 10, 16, 4, 22};  // peak, then the neighbours along dims 1, 2, 3
+      double l[7];
+#pragma unroll
+      for (int k = 0; k < 7; ++k) l[k] = __shfl_sync(0xffffffffu, lg, from[k]);
+      refine3d_from_logs(pk, l, r);
+    }
+  }
+  if (lane == 0) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) a.VF[3 * ia + d] = r[d] - a.SM[d] + g.d[d];
+  }
+}
+
+// Threads of a K3c walk block: the multiple of 32 that leaves the fewest idle
+// in the last round over P12 lag pairs (289: 160 of 320 slots a round instead
+// of 256 of 512), the larger of equal ones.
+int walk_threads(int pairs) {
+  int best = K3C_THREADS;
+  auto slots = [&](int t) { return (pairs + t - 1) / t * t; };
+  for (int t = K3C_THREADS - 32; t >= 96; t -= 32)
+    if (slots(t) < slots(best)) best = t;
+  return best;
+}
+
 template <int N, bool FPRUNE, int ALG, typename T>
 cudaError_t run_chunks(Piv3dArgs a, long long chunk, cudaStream_t s, std::string& err) {
   using L = Lay3<N, FPRUNE>;
+  constexpr bool CAN_SHARE = ALG == ALG_FFTCC || ALG == ALG_NSQECC;
+  const bool shared = CAN_SHARE && a.Gs != nullptr;
   const size_t smem = (size_t)L::SMEM_F2 * sizeof(float2);
-  cudaError_t e = cudaFuncSetAttribute(k3b_kernel<N, FPRUNE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  auto k3b = k3b_kernel<N, FPRUNE, false>;
+  if constexpr (CAN_SHARE) {
+    if (shared) k3b = k3b_kernel<N, FPRUNE, true>;
+  }
+  cudaError_t e = cudaFuncSetAttribute(k3b, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) {
     err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e);
     return e;
   }
-  const long long begin = a.ia_begin, end = a.ia_end;
+  const long long begin = a.ia_begin, end = a.ia_end, layer = (long long)a.vf[0] * a.vf[1];
+  long long l0 = 0, l1 = 0;  // layers whose z-spectra are in Gs / Fs
   constexpr int NPASS = ALG == ALG_MASK_NSQECC ? 2 : 1;
-  for (long long c0 = begin; c0 < end; c0 += chunk) {
-    const long long n = end - c0 < chunk ? end - c0 : chunk;
+  const int P12 = (2 * a.SM[0] + 1) * (2 * a.SM[1] + 1);
+  for (long long c0 = begin; c0 < end;) {
+    long long n = end - c0 < chunk ? end - c0 : chunk;
+    // as many layers as the scratch holds
+    if (shared) n = std::min(n, (c0 / layer + a.layers) * layer - c0);
     a.ia_begin = c0;
     a.ia_end = c0 + n;
     const unsigned merge_blocks = (unsigned)((n + 127) / 128);
-    for (int pass = 0; pass < NPASS; ++pass) {
-      k3a_kernel<N, FPRUNE, ALG, T><<<dim3(k3a_parts(N), (unsigned)n), K3A_THREADS, 0, s>>>(a, pass);
-      if (pass == 0) k3a_merge_kernel<N, ALG><<<merge_blocks, 128, 0, s>>>(a, n);
-      k3b_kernel<N, FPRUNE><<<dim3(L::K3, (unsigned)n), 2 * N, smem, s>>>(a, pass == 0 ? a.C : a.C2);
+    if constexpr (CAN_SHARE) {
+      if (shared) {
+        const long long f = c0 / layer, f1 = (c0 + n - 1) / layer + 1;
+        if (f < l0 || f1 > l1) {
+          l0 = f;
+          l1 = f1;
+          a.l0 = (int)l0;
+          const int th = std::min(256, (a.H + 31) / 32 * 32);
+          k3s_lines_kernel<N, FPRUNE, T><<<dim3((a.H + th - 1) / th, a.W, (unsigned)(2 * (l1 - l0))), th, 0, s>>>(a);
+        }
+        if (ALG == ALG_FFTCC && !(a.threshold >= 0.0)) {  // neither sumF2 nor a skip test
+          if ((e = cudaMemsetAsync(a.state, 0, (size_t)n * sizeof(IA3State), s)) != cudaSuccess) {
+            err = std::string("piv3d state: ") + cudaGetErrorString(e);
+            return e;
+          }
+        } else {
+          k3s_state_kernel<T, ALG><<<(unsigned)n, K3A_THREADS, 0, s>>>(a);
+        }
+      }
     }
-    const int cparts = k3c_parts(N, (2 * a.SM[0] + 1) * (2 * a.SM[1] + 1));
-    k3c_kernel<N, ALG><<<dim3(cparts, (unsigned)n), K3C_THREADS, 0, s>>>(a);
-    k3c_merge_kernel<N, ALG><<<merge_blocks, 128, 0, s>>>(a, n, cparts);
+    for (int pass = 0; pass < NPASS; ++pass) {
+      if (!shared) {
+        k3a_kernel<N, FPRUNE, ALG, T><<<dim3(k3a_parts(N), (unsigned)n), K3A_THREADS, 0, s>>>(a, pass);
+        if (pass == 0) k3a_merge_kernel<N, ALG><<<merge_blocks, 128, 0, s>>>(a, n);
+      }
+      k3b<<<dim3(L::K3, (unsigned)n), 2 * N, smem, s>>>(a, pass == 0 ? a.C : a.C2);
+    }
+    const int cparts = k3c_parts(N, P12);
+    bool done = false;
+    if constexpr (ALG != ALG_MASK_NSQECC) {
+      // without a map (batch plans) the full K3c is the faster one
+      if (finish3_fast(a, ALG) && (ALG == ALG_FFTCC || (ALG == ALG_ZNCC ? a.wz != nullptr : a.ws != nullptr))) {
+        const int th = walk_threads((P12 + cparts - 1) / cparts);
+        k3c_walk_kernel<N, ALG><<<dim3(cparts, (unsigned)n), th, 0, s>>>(a);
+        k3c_walk_merge_kernel<N, ALG><<<(unsigned)n, K3F_THREADS, 0, s>>>(a, cparts);
+        done = true;
+      }
+    }
+    if (!done) {
+      k3c_kernel<N, ALG><<<dim3(cparts, (unsigned)n), K3C_THREADS, 0, s>>>(a);
+      k3c_merge_kernel<N, ALG><<<merge_blocks, 128, 0, s>>>(a, n, cparts);
+    }
     e = cudaGetLastError();
     if (e != cudaSuccess) {
       err = std::string("piv3d launch: ") + cudaGetErrorString(e);
       return e;
     }
+    c0 += n;
   }
   return cudaSuccess;
 }
@@ -302,7 +662,7 @@ namespace {
 struct Scr3 {
   size_t b[8];
 };
-Scr3 scr3(const int IS[3], const int SM[3], int alg, size_t c) {
+Scr3 scr3(const int IS[3], const int SM[3], int alg, size_t c, bool shared) {
   Scr3 r{};
   const int SS[3] = {IS[0] + 2 * SM[0], IS[1] + 2 * SM[1], IS[2] + 2 * SM[2]};
   const int N = piv3d_fft_len(SS);
@@ -312,8 +672,8 @@ Scr3 scr3(const int IS[3], const int SM[3], int alg, size_t c) {
   const size_t P12 = (size_t)(2 * SM[0] + 1) * (2 * SM[1] + 1);
   const size_t P3 = 2 * SM[2] + 1;
   auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
-  r.b[0] = al(c * K3 * N * N * sizeof(float2));                               // Gz
-  r.b[1] = al(c * K3 * NF * NF * sizeof(float2));                             // Fz
+  r.b[0] = shared ? 0 : al(c * K3 * N * N * sizeof(float2));                  // Gz
+  r.b[1] = shared ? 0 : al(c * K3 * NF * NF * sizeof(float2));                // Fz
   r.b[2] = al(c * K3 * P12 * sizeof(float2));                                 // C
   r.b[3] = alg == ALG_MASK_NSQECC ? r.b[2] : 0;                               // C2
   r.b[4] = al(c * P12 * P3 * sizeof(float));                                  // V
@@ -324,20 +684,41 @@ Scr3 scr3(const int IS[3], const int SM[3], int alg, size_t c) {
 }
 }  // namespace
 
-size_t piv3d_scratch_bytes(const int IS[3], const int SM[3], int alg, long long chunk) {
-  const Scr3 r = scr3(IS, SM, alg, (size_t)chunk);
+size_t piv3d_scratch_bytes(const int IS[3], const int SM[3], int alg, long long chunk, bool shared) {
+  const Scr3 r = scr3(IS, SM, alg, (size_t)chunk, shared);
   size_t t = 0;
   for (size_t x : r.b) t += x;
   return t;
 }
 
-size_t piv3d_scratch_bytes_per_ia(const int IS[3], const int SM[3], int alg) {
+size_t piv3d_scratch_bytes_per_ia(const int IS[3], const int SM[3], int alg, bool shared) {
   // one IA's share, with the alignment of the eight arrays
-  return piv3d_scratch_bytes(IS, SM, alg, 1);
+  return piv3d_scratch_bytes(IS, SM, alg, 1, shared);
 }
 
-void piv3d_bind_scratch(Piv3dArgs& a, int alg, long long chunk, char* base) {
-  const Scr3 r = scr3(a.IS, a.SM, alg, (size_t)chunk);
+// Shared z-spectra (k3s_lines_kernel) of one layer, G then F; column pitches
+// are odd multiples of 128 bytes so that a window's columns spread over the
+// cache's sets.
+static long long shared3d_pitch(long long H) { return ((H + 15) / 16 | 1) * 16; }
+
+size_t piv3d_shared_bytes(const int IS[3], const int SM[3], long long H, long long W) {
+  const int SS[3] = {IS[0] + 2 * SM[0], IS[1] + 2 * SM[1], IS[2] + 2 * SM[2]};
+  const long long K3 = piv3d_fft_len(SS) / 2 + 1;
+  return (size_t)(2 * K3 * shared3d_pitch(H) * W) * sizeof(float2);
+}
+
+void piv3d_bind_shared(Piv3dArgs& a, int layers, char* base) {
+  const int SS[3] = {a.IS[0] + 2 * a.SM[0], a.IS[1] + 2 * a.SM[1], a.IS[2] + 2 * a.SM[2]};
+  a.pitch = shared3d_pitch(a.H);
+  a.zplane = a.pitch * a.W;
+  a.lstride = a.zplane * (piv3d_fft_len(SS) / 2 + 1);
+  a.layers = layers;
+  a.Gs = (float2*)base;
+  a.Fs = a.Gs + a.lstride * layers;
+}
+
+void piv3d_bind_scratch(Piv3dArgs& a, int alg, long long chunk, char* base, bool shared) {
+  const Scr3 r = scr3(a.IS, a.SM, alg, (size_t)chunk, shared);
   size_t o = 0;
   a.Gz = (float2*)(base + o);
   o += r.b[0];
@@ -354,6 +735,63 @@ void piv3d_bind_scratch(Piv3dArgs& a, int alg, long long chunk, char* base) {
   a.apart = (ReducePart3*)(base + o);
   o += r.b[6];
   a.cpart = (PeakPart3*)(base + o);
+}
+
+// Window-sum maps of a 3D pass: a thread per (i, j) and ZMAP positions along k.
+namespace {
+constexpr int ZMAP = 4;
+__device__ __forceinline__ void window_sums3(const double* __restrict__ II, int H, int W, int D, int IS3, int SM3, int r0,
+                                             int r1, int c0, int c1, int k0, int n3, double (&S)[ZMAP]) {
+#pragma unroll
+  for (int t = 0; t < ZMAP; ++t) {
+    const int k = k0 + t - SM3;
+    const int z0 = k > 0 ? k : 0, z1 = k + IS3 < D ? k + IS3 : D;
+    S[t] = k0 + t < n3 ? box_sum3(II, H, W, r0, r1, c0, c1, z0, z1) : 0.0;
+  }
+}
+__global__ void __launch_bounds__(256) window_map3_kernel(Piv3dArgs a, float2* ws, double2* wz, int n3) {
+  const int u = blockIdx.x * blockDim.x + threadIdx.x, v = blockIdx.y;
+  if (u >= a.ldw1) return;
+  const int i = u - a.SM[0], j = v - a.SM[1];
+  const int r0 = i > 0 ? i : 0, r1 = i + a.IS[0] < a.H ? i + a.IS[0] : a.H;
+  const int c0 = j > 0 ? j : 0, c1 = j + a.IS[1] < a.W ? j + a.IS[1] : a.W;
+  const int k0 = blockIdx.z * ZMAP;
+  double S2[ZMAP], S1[ZMAP];
+  window_sums3(a.IIg2, a.H, a.W, a.D, a.IS[2], a.SM[2], r0, r1, c0, c1, k0, n3, S2);
+  if (wz) window_sums3(a.IIg, a.H, a.W, a.D, a.IS[2], a.SM[2], r0, r1, c0, c1, k0, n3, S1);
+#pragma unroll
+  for (int t = 0; t < ZMAP; ++t) {
+    if (k0 + t < n3) {
+      const long long at = u + (long long)a.ldw1 * (v + (long long)a.ldw2 * (k0 + t));
+      if (wz) {
+        wz[at] = make_double2(S2[t], S1[t]);
+      } else {
+        const float q = (float)S2[t];
+        ws[at] = make_float2(q, sqrtf(q));
+      }
+    }
+  }
+}
+}  // namespace
+
+size_t window_map3_bytes(const Piv3dArgs& a, int alg) {
+  const size_t n = (size_t)winmap_ld(a.H, a.IS[0], a.SM[0]) * (size_t)winmap_ld(a.W, a.IS[1], a.SM[1]) *
+                   (size_t)winmap_ld(a.D, a.IS[2], a.SM[2]);
+  return n * (alg == ALG_ZNCC ? sizeof(double2) : sizeof(float2));
+}
+
+cudaError_t launch_window_map3(Piv3dArgs& a, int alg, void* base, cudaStream_t s) {
+  a.ldw1 = winmap_ld(a.H, a.IS[0], a.SM[0]);
+  a.ldw2 = winmap_ld(a.W, a.IS[1], a.SM[1]);
+  const int n3 = winmap_ld(a.D, a.IS[2], a.SM[2]);
+  if (a.ldw2 > 65535 || (n3 + ZMAP - 1) / ZMAP > 65535) return cudaSuccess;  // no map: the integral volumes are read
+  float2* ws = alg == ALG_ZNCC ? nullptr : (float2*)base;
+  double2* wz = alg == ALG_ZNCC ? (double2*)base : nullptr;
+  const int th = std::min(256, (a.ldw1 + 31) / 32 * 32);
+  window_map3_kernel<<<dim3((a.ldw1 + th - 1) / th, a.ldw2, (n3 + ZMAP - 1) / ZMAP), th, 0, s>>>(a, ws, wz, n3);
+  a.ws = ws;
+  a.wz = wz;
+  return cudaGetLastError();
 }
 
 cudaError_t launch_piv3d(const Piv3dArgs& a, int alg, long long chunk, cudaStream_t s, std::string& err) {

@@ -84,6 +84,15 @@ struct Piv3dArgs {
   IA3State* state;        // [ci]
   ReducePart3* apart;     // [ci][k3a_parts(N)]
   PeakPart3* cpart;       // [ci][k3c_parts(N, P1 P2)]
+  // z-spectra shared by the IAs of a layer (k3s_*), or null: Gz / Fz per IA
+  float2* Gs;             // [layer - l0][k3][x2][x1] over the image, column pitch `pitch`
+  float2* Fs;
+  long long pitch, zplane, lstride;  // float2 between x2 columns, k3 planes, layers
+  int l0, layers;         // first layer of the chunk, layers the scratch holds
+  // window-sum maps (mqp_finish3.cuh), or null: read the integral volumes
+  const float2* ws;       // NSQECC: (S2, sqrt S2)
+  const double2* wz;      // ZNCC: (S2, S1)
+  int ldw1, ldw2;         // extents along dims 1 and 2
 };
 
 template <int N, bool FPRUNE>
@@ -328,6 +337,50 @@ MQP_HD MQP_FI void k3b_rows(const Piv3dArgs& a, const IAGeom3& g, long long ci, 
       for (int n = 0; n < M; ++n) {
         const float2 u = (n < L::NF && n < a.IS[1]) ? src[n * L::NF] : z0;
         const float2 v = (n + M < L::NF && n + M < a.IS[1]) ? src[(n + M) * L::NF] : z0;
+        y[n] = dif_in<N>(h, n, u, v);
+      }
+      fft_reg<M, false>(y);
+#pragma unroll
+      for (int m = 0; m < M; ++m) SF[(2 * m + h) * L::FSTR + t] = y[fpos<M>(m)];
+    } else {
+#pragma unroll 4
+      for (int m = 0; m < M; ++m) SF[(2 * m + h) * L::FSTR + t] = z0;
+    }
+  }
+}
+
+// Phase R from the layer's shared z-spectra: the IA's windows are read out of
+// the image-wide planes.
+template <int N, bool FPRUNE>
+MQP_HD MQP_FI void k3b_rows_shared(const Piv3dArgs& a, const IAGeom3& g, int k3, int t, int h, float2* S, float2* SF) {
+  using L = Lay3<N, FPRUNE>;
+  constexpr int M = N / 2;
+  const long long plane = k3 * a.zplane + (g.v[2] - a.l0) * a.lstride;
+  const float2 z0 = make_float2(0.f, 0.f);
+  if (t >= g.lo[0] && t < g.hi[0]) {
+    const float2* src = a.Gs + (plane + (g.g0[0] + t) + a.pitch * g.g0[1]);
+    float2 y[M];
+#pragma unroll
+    for (int n = 0; n < M; ++n) {
+      const float2 u = (n >= g.lo[1] && n < g.hi[1]) ? src[n * a.pitch] : z0;
+      const float2 v = (n + M >= g.lo[1] && n + M < g.hi[1]) ? src[(n + M) * a.pitch] : z0;
+      y[n] = dif_in<N>(h, n, u, v);
+    }
+    fft_reg<M, false>(y);
+#pragma unroll
+    for (int m = 0; m < M; ++m) S[(2 * m + h) * L::SSTR + t] = y[fpos<M>(m)];
+  } else {
+#pragma unroll 4
+    for (int m = 0; m < M; ++m) S[(2 * m + h) * L::SSTR + t] = z0;
+  }
+  if (t < L::NF) {
+    if (t < a.IS[0]) {
+      const float2* src = a.Fs + (plane + (g.ir[0] + t) + a.pitch * g.ir[1]);
+      float2 y[M];
+#pragma unroll
+      for (int n = 0; n < M; ++n) {
+        const float2 u = (n < L::NF && n < a.IS[1]) ? src[n * a.pitch] : z0;
+        const float2 v = (n + M < L::NF && n + M < a.IS[1]) ? src[(n + M) * a.pitch] : z0;
         y[n] = dif_in<N>(h, n, u, v);
       }
       fft_reg<M, false>(y);
