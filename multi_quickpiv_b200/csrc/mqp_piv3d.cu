@@ -217,24 +217,26 @@ __global__ void __launch_bounds__(2 * N) k3b_kernel(Piv3dArgs a, float2* C) {
     float2 p[M];
     k3b_cols_f<N, FPRUNE>(t, h, S, SF, p);
     __syncthreads();
-    k3b_x1<N, FPRUNE>(t, h, p, S);
-  }
-  __syncthreads();
-  {
+    k3b_x1<N, FPRUNE>(t, h, p, S, P1);
+    __syncthreads();
     float2 o[M];
-    k3b_x2<N, FPRUNE>(t, h, S, o);
+    k3b_x2<N, FPRUNE>(t, h, S, o, P1, p);
     __syncthreads();
     k3b_x3<N, FPRUNE>(t, h, P1, o, S);
   }
   __syncthreads();
   {
+    // the 2 P1 half rows go to consecutive threads: at 33 lags three warps
+    // work where (t, h) would take all four for two of their lanes
+    const int t2 = threadIdx.x % P1, h2 = threadIdx.x / P1;  // P1 <= N
+    const int tr = h2 < 2 ? t2 : P1;
     float2 u[M];
-    k3b_r2a<N, FPRUNE>(t, h, P1, S, u);
+    k3b_r2a<N, FPRUNE>(tr, h2, P1, S, u);
     __syncthreads();
-    k3b_r2b<N, FPRUNE>(t, h, P1, u, S);
+    k3b_r2b<N, FPRUNE>(tr, h2, P1, u, S, P2);
+    __syncthreads();
+    k3b_r2c<N, FPRUNE>(ci, k3, tr, h2, P1, P2, S, C, u);
   }
-  __syncthreads();
-  k3b_r2c<N, FPRUNE>(ci, k3, t, h, P1, P2, S, C);
 }
 
 // Blocks (part, IA): each part walks its contiguous share of the lag pairs;

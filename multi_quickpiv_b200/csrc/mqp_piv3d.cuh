@@ -436,25 +436,34 @@ MQP_HD MQP_FI void k3b_cols_f(int t, int h, const float2* S, const float2* SF, f
 // Exchange of a pair's inverse halves through column t of T (T aliases S):
 // X1 writes z_0[n] (h = 0) or W_N^-n z_1[n] (h = 1) to row n + hM; X2 (after a
 // barrier) reads both and keeps x[n + hM] = z_0[n] +- W_N^-n z_1[n]; X3 (after
-// a barrier) stores the lags s1 < P1 to T[s1][t].
+// a barrier) stores the lags s1 < P1 to T[s1][t].  Only what the kept lags need
+// moves: thread (t, 0) has z_0 itself (p: its inverse, still in registers) and
+// leaves the few of its values that the lags past M need, thread (t, 1) reads
+// and forms only those.
 template <int N, bool FPRUNE>
-MQP_HD MQP_FI void k3b_x1(int t, int h, const float2 (&p)[N / 2], float2* T) {
+MQP_HD MQP_FI void k3b_x1(int t, int h, const float2 (&p)[N / 2], float2* T, int P1 = N) {
   using L = Lay3<N, FPRUNE>;
   constexpr int M = N / 2;
+  if (h) {
 #pragma unroll
-  for (int n = 0; n < M; ++n) {
-    const float2 w = p[fpos<M>(n)];
-    T[(n + h * M) * L::SSTR + t] = h ? rotate<N, true>(w, n) : w;
+    for (int n = 0; n < M; ++n) T[(n + M) * L::SSTR + t] = rotate<N, true>(p[fpos<M>(n)], n);
+  } else {
+#pragma unroll
+    for (int n = 0; n < M; ++n)
+      if (n + M < P1) T[n * L::SSTR + t] = p[fpos<M>(n)];
   }
 }
 template <int N, bool FPRUNE>
-MQP_HD MQP_FI void k3b_x2(int t, int h, const float2* T, float2 (&o)[N / 2]) {
+MQP_HD MQP_FI void k3b_x2(int t, int h, const float2* T, float2 (&o)[N / 2], int P1 = N, const float2* p = nullptr) {
   using L = Lay3<N, FPRUNE>;
   constexpr int M = N / 2;
+  if (h) {
 #pragma unroll
-  for (int n = 0; n < M; ++n) {
-    const float2 a = T[n * L::SSTR + t], b = T[(n + M) * L::SSTR + t];
-    o[n] = h ? csub(a, b) : cadd(a, b);
+    for (int n = 0; n < M; ++n)
+      if (n + M < P1) o[n] = csub(T[n * L::SSTR + t], T[(n + M) * L::SSTR + t]);
+  } else {
+#pragma unroll
+    for (int n = 0; n < M; ++n) o[n] = cadd(p ? p[fpos<M>(n)] : T[n * L::SSTR + t], T[(n + M) * L::SSTR + t]);
   }
 }
 template <int N, bool FPRUNE>
@@ -469,7 +478,8 @@ MQP_HD MQP_FI void k3b_x3(int t, int h, int P1, const float2 (&o)[N / 2], float2
 // Phase R2a: thread (s1 = t < P1, h) takes the bins k2 of parity h of lag row
 // s1 and inverts them (M points); R2b (after a barrier) writes its half to
 // the row; R2c (after a barrier) combines the halves into lags s2 = n + hM
-// and stores those below P2 to C[ci][k3][s2][s1].
+// and stores those below P2 to C[ci][k3][s2][s1]; the exchange moves what
+// the kept lags need, as above.
 template <int N, bool FPRUNE>
 MQP_HD MQP_FI void k3b_r2a(int t, int h, int P1, const float2* T, float2 (&u)[N / 2]) {
   using L = Lay3<N, FPRUNE>;
@@ -480,29 +490,34 @@ MQP_HD MQP_FI void k3b_r2a(int t, int h, int P1, const float2* T, float2 (&u)[N 
   fft_reg<M, true>(u);
 }
 template <int N, bool FPRUNE>
-MQP_HD MQP_FI void k3b_r2b(int t, int h, int P1, const float2 (&u)[N / 2], float2* T) {
+MQP_HD MQP_FI void k3b_r2b(int t, int h, int P1, const float2 (&u)[N / 2], float2* T, int P2 = N) {
   using L = Lay3<N, FPRUNE>;
   constexpr int M = N / 2;
   if (t >= P1) return;
+  if (h) {
 #pragma unroll
-  for (int n = 0; n < M; ++n) {
-    const float2 w = u[fpos<M>(n)];
-    T[t * L::SSTR + n + h * M] = h ? rotate<N, true>(w, n) : w;
+    for (int n = 0; n < M; ++n) T[t * L::SSTR + n + M] = rotate<N, true>(u[fpos<M>(n)], n);
+  } else {
+#pragma unroll
+    for (int n = 0; n < M; ++n)
+      if (n + M < P2) T[t * L::SSTR + n] = u[fpos<M>(n)];
   }
 }
 template <int N, bool FPRUNE>
-MQP_HD MQP_FI void k3b_r2c(long long ci, int k3, int t, int h, int P1, int P2, const float2* T, float2* C) {
+MQP_HD MQP_FI void k3b_r2c(long long ci, int k3, int t, int h, int P1, int P2, const float2* T, float2* C,
+                           const float2* p = nullptr) {
   using L = Lay3<N, FPRUNE>;
   constexpr int M = N / 2;
   if (t >= P1) return;
   float2* dst = C + ((ci * L::K3 + k3) * P2) * (long long)P1 + t;
+  if (h) {
 #pragma unroll
-  for (int n = 0; n < M; ++n) {
-    const int s2 = n + h * M;
-    if (s2 < P2) {
-      const float2 a = T[t * L::SSTR + n], b = T[t * L::SSTR + n + M];
-      dst[(long long)s2 * P1] = h ? csub(a, b) : cadd(a, b);
-    }
+    for (int n = 0; n < M; ++n)
+      if (n + M < P2) dst[(long long)(n + M) * P1] = csub(T[t * L::SSTR + n], T[t * L::SSTR + n + M]);
+  } else {
+#pragma unroll
+    for (int n = 0; n < M; ++n)
+      if (n < P2) dst[(long long)n * P1] = cadd(p ? p[fpos<M>(n)] : T[t * L::SSTR + n], T[t * L::SSTR + n + M]);
   }
 }
 
