@@ -9,10 +9,11 @@
 //            through one 64-point complex FFT (r2c_store); spectra rows
 //            k2 = 0..63 go to shared memory, k2 = 0 and k2 = 64 (both real)
 //            packed as one complex row.
-//   columns  lanes (2c, 2c+1) own spectrum column c: a first radix-2 DIF
+//   columns  threads (c, c + 64) own spectrum column c: a first radix-2 DIF
 //            stage splits each 128-point column transform into its even and
-//            odd bins, one 64-point FFT per lane, for G and F; conj(F) G; the
-//            64-point inverses are recombined as
+//            odd bins (the first and the second 64 threads, so that a warp
+//            takes one side of the split), one 64-point FFT per thread, for G
+//            and F; conj(F) G; the 64-point inverses are recombined as
 //              x[s] = A0[s] + W^-s A1[s],  x[s+64] = A0[s] - W^-s A1[s]
 //            with the partner's half read through the pair's own row of
 //            shared memory.  Lags s1 < P1 stay.
@@ -69,25 +70,37 @@ template <bool FPRUNE, typename T, int ALG>
 MQP_PHASE void big_rows(const Piv2dArgs& a, const IAGeom& g, const IAScalars& sc, int PASS, int t, float2* S,
                         float2* SF, double& vmax, double& mmax, double& sumsq) {
   using L = LayBig<FPRUNE>;
+  // Every row's pixels are loaded half a row at a time before any is used, at
+  // addresses clamped into the row (no branch per pixel): loaded one by one
+  // under their conditions they cost a round trip each, two fifths of the kernel.
+  constexpr int RB = MB;
   {  // G row t
     float2 z[MB];
-    const bool live = t >= g.lo1 && t < g.hi1;
+    const bool live = t >= g.lo1 && t < g.hi1 && g.hi2 > g.lo2;
     if (live) {
       const T* p = reinterpret_cast<const T*>(a.img2) + ((long long)(g.g01 + t) + (long long)a.H * g.g02);
       const float mg = (float)sc.meanG;
-      float w[NB];
+      const int lo2 = g.lo2, hi2 = g.hi2;
+      const long long H = a.H;
 #pragma unroll
-      for (int x = 0; x < NB; ++x) {
-        w[x] = 0.f;
-        if (x >= g.lo2 && x < g.hi2) {
-          float v = (float)ldg_px<T>(p, (long long)a.H * x);
+      for (int b = 0; b < NB; b += RB) {
+        T raw[RB];
+#pragma unroll
+        for (int x = 0; x < RB; ++x) {
+          const int c = b + x < lo2 ? lo2 : (b + x < hi2 ? b + x : hi2 - 1);
+          raw[x] = ldg_px<T>(p, H * c);
+        }
+        mqp_no_hoist();
+#pragma unroll
+        for (int x = 0; x < RB; ++x) {
+          float v = (float)raw[x];
           if (ALG == ALG_ZNCC) v = v - mg;
           if (PASS == PASS_MASK_SQ) v = v * v;
-          w[x] = v;
+          v = (b + x >= lo2 && b + x < hi2) ? v : 0.f;
+          if (x & 1) z[(b + x) / 2].y = v;
+          else z[(b + x) / 2].x = v;
         }
       }
-#pragma unroll
-      for (int n = 0; n < MB; ++n) z[n] = make_float2(w[2 * n], w[2 * n + 1]);
       r2c_store<NB, MB>(z, S + t, L::SSTR);
     } else {
       zero_strided(S + t, MB, L::SSTR);
@@ -103,46 +116,64 @@ MQP_PHASE void big_rows(const Piv2dArgs& a, const IAGeom& g, const IAScalars& sc
     const T* p = reinterpret_cast<const T*>(a.img1) + base;
     const T* q = PASS != PASS_PLAIN ? reinterpret_cast<const T*>(a.mask) + base : p;
     const T* qs = PASS == PASS_MASKED ? reinterpret_cast<const T*>(a.mask_skip ? a.mask_skip : a.mask) + base : p;
-    float w[NB];
+    float2 z[MB];
+    const int IS2 = a.IS2;
+    const long long H = a.H;
+    double vm = vmax, mm = mmax, ss = sumsq;
+    // masked NSQECC reads three images: a quarter row at a time
+    constexpr int FB = ALG == ALG_MASK_NSQECC ? RB / 2 : RB;
 #pragma unroll
-    for (int x = 0; x < NB; ++x) {
-      w[x] = 0.f;
-      if (x < L::NF && x < a.IS2) {
-        const long long off = (long long)a.H * x;
-        if (PASS == PASS_PLAIN) {
-          const T r = ldg_px<T>(p, off);
-          vmax = (double)r > vmax ? (double)r : vmax;
-          const double val = (double)r - sc.meanF;
-          sumsq += val * val;
-          w[x] = (float)val;
-        } else if (PASS == PASS_MASKED) {
-          const T r = ldg_px<T>(p, off);
-          const T mk = ldg_px<T>(q, off);
-          const T ms = ldg_px<T>(qs, off);
-          vmax = (double)r > vmax ? (double)r : vmax;
-          mmax = (double)ms > mmax ? (double)ms : mmax;
-          const double val = (double)r * (double)mk;
-          sumsq += val * val / ((double)mk > 0.0 ? (double)mk : 1.0);
-          w[x] = (float)val;
-        } else {
-          w[x] = (float)ldg_px<T>(q, off);
+    for (int b = 0; b < NB; b += FB) {
+      T raw[FB], mk[FB], ms[FB];
+#pragma unroll
+      for (int x = 0; x < FB; ++x) {
+        const long long off = H * (b + x < IS2 ? b + x : IS2 - 1);
+        raw[x] = mk[x] = ms[x] = T(0);
+        if (b + x < L::NF) {
+          if (PASS != PASS_MASK_SQ) raw[x] = ldg_px<T>(p, off);
+          if (ALG == ALG_MASK_NSQECC) mk[x] = ldg_px<T>(q, off);
+          if (ALG == ALG_MASK_NSQECC && PASS == PASS_MASKED) ms[x] = ldg_px<T>(qs, off);
         }
       }
-    }
-    float2 z[MB];
+      mqp_no_hoist();
 #pragma unroll
-    for (int n = 0; n < MB; ++n) z[n] = make_float2(w[2 * n], w[2 * n + 1]);
+      for (int x = 0; x < FB; ++x) {
+        float w = 0.f;
+        if (b + x < L::NF && b + x < IS2) {
+          if (PASS == PASS_PLAIN) {
+            const T r = raw[x];
+            vm = (double)r > vm ? (double)r : vm;
+            const double val = (double)r - sc.meanF;
+            ss += val * val;
+            w = (float)val;
+          } else if (PASS == PASS_MASKED) {
+            vm = (double)raw[x] > vm ? (double)raw[x] : vm;
+            mm = (double)ms[x] > mm ? (double)ms[x] : mm;
+            const double val = (double)raw[x] * (double)mk[x];
+            ss += val * val / ((double)mk[x] > 0.0 ? (double)mk[x] : 1.0);
+            w = (float)val;
+          } else {
+            w = (float)mk[x];
+          }
+        }
+        if (x & 1) z[(b + x) / 2].y = w;
+        else z[(b + x) / 2].x = w;
+      }
+    }
+    vmax = vm;
+    mmax = mm;
+    sumsq = ss;
     r2c_store<NB, FPRUNE ? MB / 2 : MB>(z, out, L::FSTR);
   }
 }
 
 // ---- columns ----------------------------------------------------------------
-// Step 1 (lane t: column c = t/2, half h = t%2): the DIF split and 64-point
+// Step 1 (thread t: column c = t % 64, half h = t / 64): the DIF split and 64-point
 // FFT of G column c; y[fpos(m)] = bin 2m+h.
 template <bool FPRUNE>
 MQP_HD MQP_FI void big_col_g(int t, const float2* S, float2 (&y)[MB]) {
   using L = LayBig<FPRUNE>;
-  const int c = t >> 1, h = t & 1;
+  const int c = t & (MB - 1), h = t / MB;
   const float2* row = S + c * L::SSTR;
   if (h) {
 #pragma unroll
@@ -159,7 +190,7 @@ MQP_HD MQP_FI void big_col_g(int t, const float2* S, float2 (&y)[MB]) {
 template <bool FPRUNE>
 MQP_HD MQP_FI void big_col_park(int t, const float2 (&y)[MB], float2* S) {
   using L = LayBig<FPRUNE>;
-  const int c = t >> 1, h = t & 1;
+  const int c = t & (MB - 1), h = t / MB;
   float2* row = S + c * L::SSTR + MB * h;
 #pragma unroll
   for (int m = 0; m < MB; ++m) row[m] = y[fpos<MB>(m)];
@@ -174,7 +205,7 @@ MQP_HD MQP_FI void big_col_park(int t, const float2 (&y)[MB], float2* S) {
 template <bool FPRUNE>
 MQP_HD MQP_FI void big_col_product(int t, const float2* S, const float2* SF, float2* PK, float2 (&p)[MB]) {
   using L = LayBig<FPRUNE>;
-  const int c = t >> 1, h = t & 1;
+  const int c = t & (MB - 1), h = t / MB;
   const float2* frow = SF + c * L::FSTR;
   const float2* G = S + c * L::SSTR + MB * h;
   float2 f[MB];
@@ -187,6 +218,41 @@ MQP_HD MQP_FI void big_col_product(int t, const float2* S, const float2* SF, flo
     for (int n = 0; n < MB; ++n) f[n] = (L::NF > MB) ? cadd(frow[n], frow[n + MB]) : frow[n];
   }
   fft_reg<MB, false>(f);
+#if defined(__CUDA_ARCH__)
+  // the warp of column 0 forms its 64 products together, two a lane (by itself
+  // the column's thread would hold the block up for some 3,000 instructions)
+  if (c == 0) {
+    float2* F = PK + MB * h;
+#pragma unroll
+    for (int m = 0; m < MB; ++m) F[m] = f[fpos<MB>(m)];
+  }
+  if (c < 32) {
+    __syncwarp();
+    const float2* F = PK + MB * h;
+    const float2* G0 = S + MB * h;
+    float2 q[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int m = (t & 31) + 32 * k;
+      const int mm = h ? MB - 1 - m : (MB - m) & (MB - 1);
+      const float2 Zk = G0[m], Zn = cconj(G0[mm]);
+      const float2 Fk = F[m], Fn = cconj(F[mm]);
+      const float2 A = cscale(cadd(Zk, Zn), 0.5f), B = cscale(cmul_mi(csub(Zk, Zn)), 0.5f);
+      const float2 Af = cscale(cadd(Fk, Fn), 0.5f), Bf = cscale(cmul_mi(csub(Fk, Fn)), 0.5f);
+      q[k] = cadd(cmulc(Af, A), cmul_pi(cmulc(Bf, B)));
+    }
+    __syncwarp();
+    PK[MB * h + (t & 31)] = q[0];
+    PK[MB * h + (t & 31) + 32] = q[1];
+    __syncwarp();
+  }
+#pragma unroll
+  for (int m = 0; m < MB; ++m) p[m] = cmulc(f[fpos<MB>(m)], G[m]);
+  if (c == 0) {
+#pragma unroll
+    for (int m = 0; m < MB; ++m) p[m] = PK[MB * h + m];
+  }
+#else
   if (c != 0) {
 #pragma unroll
     for (int m = 0; m < MB; ++m) p[m] = cmulc(f[fpos<MB>(m)], G[m]);
@@ -204,6 +270,7 @@ MQP_HD MQP_FI void big_col_product(int t, const float2* S, const float2* SF, flo
       p[m] = cadd(cmulc(Af, A), cmul_pi(cmulc(Bf, B)));
     }
   }
+#endif
   fft_reg<MB, true>(p);
 }
 
@@ -220,7 +287,7 @@ MQP_HD MQP_FI void big_col_park_a(int t, const float2 (&p)[MB], float2* S) {
 template <bool FPRUNE>
 MQP_HD MQP_FI void big_col_combine(int t, int P1, const float2* S, float2 (&out)[MB]) {
   using L = LayBig<FPRUNE>;
-  const int c = t >> 1, h = t & 1;
+  const int c = t & (MB - 1), h = t / MB;
   const float2* row = S + c * L::SSTR;
   const int n = P1 - MB * h;  // lags this lane keeps
 #pragma unroll
@@ -237,7 +304,7 @@ MQP_HD MQP_FI void big_col_combine(int t, int P1, const float2* S, float2 (&out)
 template <bool FPRUNE>
 MQP_HD MQP_FI void big_col_store(int t, int P1, const float2 (&out)[MB], float2* T) {
   using L = LayBig<FPRUNE>;
-  const int c = t >> 1, h = t & 1;
+  const int c = t & (MB - 1), h = t / MB;
   const int n = P1 - MB * h;
 #pragma unroll
   for (int s = 0; s < MB; ++s)
@@ -252,7 +319,7 @@ template <bool FPRUNE>
 __device__ __noinline__ void big_columns_g(int t, float2* S) {
   float2 y[MB];
   big_col_g<FPRUNE>(t, S, y);
-  __syncwarp();
+  __syncthreads();
   big_col_park<FPRUNE>(t, y, S);
 }
 template <bool FPRUNE>
@@ -272,7 +339,7 @@ template <bool FPRUNE>
 __device__ __forceinline__ void big_columns(int t, int P1, float2* S, const float2* SF, float2* PK) {
   big_columns_g<FPRUNE>(t, S);
   big_columns_product<FPRUNE>(t, S, SF, PK);
-  __syncwarp();
+  __syncthreads();
   big_columns_combine<FPRUNE>(t, P1, S);
 }
 #endif
