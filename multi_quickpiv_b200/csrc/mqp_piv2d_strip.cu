@@ -24,9 +24,9 @@
 // Bound by instruction issue and supply: 9.5k warp instructions per IA (15.3k
 // before), issue active 45 %, stalls led by no_instruction (1.25 warps per
 // issue) and the barrier after the rows (1.07).  Measured on B200 (kernel,
-// one warp per IA -> strips): 2048^2 NSQECC step 8 2113 -> 1403 us, FFTCC 1270 ->
-// 1197; 1024x1280 NSQECC step 16 199 -> 106; 2048^2 NSQECC step 16 with SN 589 ->
-// 432; 256^2 FFTCC Float64 step 16 35 -> 23.
+// one warp per IA -> strips): 2048^2 NSQECC step 8 2113 -> 1202 us, FFTCC 1270 ->
+// 1023; 1024x1280 NSQECC step 16 199 -> 93; 2048^2 NSQECC step 16 with SN 589 ->
+// 354; 256^2 FFTCC Float64 step 16 35 -> 17.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -45,8 +45,8 @@ constexpr int SN_ = 64;            // FFT length
 constexpr int SM_ = SN_ / 2;       // spectrum columns per IA: one per lane
 // Four warps, three blocks to an SM (168 registers): twelve warps.  Measured on
 // the 2048^2 NSQECC pass at step 8: 1403 us so, 1775 with four (128 registers,
-// 1.5 KB of spill), 1592 with two (255
-// registers, no spill), 1653 with one block of eight warps and IAs; block
+// 1.5 KB of spill), 1592 with two (255 registers, no spill), 1653 with one
+// block of eight warps and IAs (all before the rows loaded in batches); block
 // sizes that are not a multiple of four warps load the SM's quarters unevenly.
 constexpr int STRIP_WARPS = 4, STRIP_BLOCKS = 3;
 constexpr size_t STRIP_SMEM = 220 * 1024;  // of the 227 KB a block can have
@@ -96,17 +96,26 @@ __device__ __forceinline__ void pair_barrier(int id) {
 template <typename T>
 __device__ __forceinline__ void strip_row(const Piv2dArgs& a, const IAGeom& g, bool isF, long long base, float2* out,
                                           int stride, double2* red) {
+  // loads in batches at addresses clamped into the row, before any is used: one
+  // by one under their conditions they cost a round trip each (2048^2 NSQECC
+  // step 8 1403 -> 1202 us, step 16 with SN 432 -> 354)
   float2 z[SM_];
+  const long long H = a.H;
+  constexpr int RB = SM_;
   if (isF) {
     const T* p = reinterpret_cast<const T*>(a.img1) + base;
+    const int IS2 = a.IS2;
+    T raw[RB];
+#pragma unroll
+    for (int x = 0; x < RB; ++x) raw[x] = ldg_px<T>(p, H * (x < IS2 ? x : IS2 - 1));
+    mqp_no_hoist();
     double vmax = -INFINITY, sumsq = 0.0;
 #pragma unroll
-    for (int x = 0; x < SM_; ++x) {
+    for (int x = 0; x < RB; ++x) {
       float w = 0.f;
-      if (x < a.IS2) {
-        const T r = ldg_px<T>(p, (long long)a.H * x);
-        vmax = (double)r > vmax ? (double)r : vmax;
-        const double val = (double)r;
+      if (x < IS2) {
+        const double val = (double)raw[x];
+        vmax = val > vmax ? val : vmax;
         sumsq += val * val;
         w = (float)val;
       }
@@ -114,15 +123,26 @@ __device__ __forceinline__ void strip_row(const Piv2dArgs& a, const IAGeom& g, b
       else z[x / 2].x = w;
     }
 #pragma unroll
-    for (int n = SM_ / 2; n < SM_; ++n) z[n] = make_float2(0.f, 0.f);
+    for (int n = RB / 2; n < SM_; ++n) z[n] = make_float2(0.f, 0.f);
     *red = make_double2(vmax, sumsq);
   } else {
     const T* p = reinterpret_cast<const T*>(a.img2) + base;
+    const int lo2 = g.lo2, hi2 = g.hi2;
 #pragma unroll
-    for (int n = 0; n < SM_; ++n) {
-      const int x0 = 2 * n, x1 = 2 * n + 1;
-      z[n] = make_float2((x0 >= g.lo2 && x0 < g.hi2) ? (float)ldg_px<T>(p, (long long)a.H * x0) : 0.f,
-                         (x1 >= g.lo2 && x1 < g.hi2) ? (float)ldg_px<T>(p, (long long)a.H * x1) : 0.f);
+    for (int b = 0; b < SN_; b += RB) {
+      T raw[RB];
+#pragma unroll
+      for (int x = 0; x < RB; ++x) {
+        const int c = b + x < lo2 ? lo2 : (b + x < hi2 ? b + x : hi2 - 1);
+        raw[x] = ldg_px<T>(p, H * c);
+      }
+      if (sizeof(T) == 8) mqp_no_hoist();
+#pragma unroll
+      for (int x = 0; x < RB; ++x) {
+        const float v = (b + x >= lo2 && b + x < hi2) ? (float)raw[x] : 0.f;
+        if (x & 1) z[(b + x) / 2].y = v;
+        else z[(b + x) / 2].x = v;
+      }
     }
   }
   r2c_store<SN_, SM_>(z, out, stride);
@@ -651,7 +671,7 @@ cudaError_t launch_piv2d_strip(const Piv2dArgs& a, int alg, cudaStream_t s, std:
   // Strips of four fill the SMs from STRIP_BLOCKS blocks of four IAs each;
   // a pass of no more IAs than blocks takes two warps to an IA instead.
   // Measured (kernel): 225 IAs 20.9 us in strips of four, 18.6 as pairs of
-  // warps; 256 IAs (interSize 32, margin 10) 36 and 27 us.
+  // warps; 256 IAs (interSize 32, margin 10) 36 and 27 us (now 17 and 23).
   const int wpi = n_ia <= (long long)STRIP_BLOCKS * sms ? 2 : 1;
   int n = wpi == 2 ? 1 : 4;
   StripCfg c = strip_cfg(a, n, wpi);

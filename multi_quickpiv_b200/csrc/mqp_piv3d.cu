@@ -120,8 +120,14 @@ __global__ void __launch_bounds__(256) k3s_lines_kernel(Piv3dArgs a) {
 #pragma unroll
     for (int n = 0; n < M; ++n) {
       const int u = 2 * n, v = 2 * n + 1;
-      z[n] = make_float2(u < FLIM && u < a.IS[2] ? (float)ldg_px<T>(p, HW * u) : 0.f,
-                         v < FLIM && v < a.IS[2] ? (float)ldg_px<T>(p, HW * v) : 0.f);
+      z[n] = make_float2(0.f, 0.f);
+      if (u < FLIM) z[n].x = (float)ldg_px<T>(p, HW * min(u, a.IS[2] - 1));
+      if (v < FLIM) z[n].y = (float)ldg_px<T>(p, HW * min(v, a.IS[2] - 1));
+    }
+#pragma unroll
+    for (int n = 0; n < M; ++n) {
+      if (2 * n >= a.IS[2]) z[n].x = 0.f;
+      if (2 * n + 1 >= a.IS[2]) z[n].y = 0.f;
     }
     r2c_line_store<N, FPRUNE ? M / 2 : M>(z, out, a.zplane);
   } else {
@@ -130,8 +136,12 @@ __global__ void __launch_bounds__(256) k3s_lines_kernel(Piv3dArgs a) {
 #pragma unroll
     for (int n = 0; n < M; ++n) {
       const int u = 2 * n, v = 2 * n + 1;
-      z[n] = make_float2(u >= zl && u < zh ? (float)ldg_px<T>(p, HW * u) : 0.f,
-                         v >= zl && v < zh ? (float)ldg_px<T>(p, HW * v) : 0.f);
+      z[n] = make_float2((float)ldg_px<T>(p, HW * min(max(u, zl), zh - 1)), (float)ldg_px<T>(p, HW * min(max(v, zl), zh - 1)));
+    }
+#pragma unroll
+    for (int n = 0; n < M; ++n) {
+      if (2 * n < zl || 2 * n >= zh) z[n].x = 0.f;
+      if (2 * n + 1 < zl || 2 * n + 1 >= zh) z[n].y = 0.f;
     }
     r2c_line_store<N, M>(z, out, a.zplane);
   }

@@ -225,29 +225,44 @@ MQP_HD MQP_FI void k3a_line(const Piv3dArgs& a, const IAGeom3& g, const IA3State
     const T* q = PASS != PASS_PLAIN ? reinterpret_cast<const T*>(a.mask) + base : p;
     const T* qs = PASS == PASS_MASKED ? reinterpret_cast<const T*>(a.mask_skip ? a.mask_skip : a.mask) + base : p;
     constexpr int FLIM = L::NF;  // z extent an IA line can occupy
+    // loaded FB at a time before any is used, at addresses clamped into the line
+    constexpr int FB = FLIM < 32 ? FLIM : 32;
+    const int IS3 = a.IS[2];
 #pragma unroll
-    for (int x = 0; x < N; ++x) {
-      w[x] = 0.f;
-      if (x < FLIM && x < a.IS[2]) {
-        const long long off = HW * x;
-        if (PASS == PASS_PLAIN) {
-          const T r = ldg_px<T>(p, off);
-          vmax = (double)r > vmax ? (double)r : vmax;
-          const double val = (double)r - s.meanF;
-          sumsq += val * val;
-          w[x] = (float)val;
-        } else if (PASS == PASS_MASKED) {
-          const T r = ldg_px<T>(p, off);
-          const T mk = ldg_px<T>(q, off);
-          const T ms = ldg_px<T>(qs, off);
-          vmax = (double)r > vmax ? (double)r : vmax;
-          mmax = (double)ms > mmax ? (double)ms : mmax;
-          const double val = (double)r * (double)mk;
-          sumsq += val * val / ((double)mk > 0.0 ? (double)mk : 1.0);
-          w[x] = (float)val;
-        } else {
-          w[x] = (float)ldg_px<T>(q, off);
+    for (int x = FLIM; x < N; ++x) w[x] = 0.f;
+#pragma unroll
+    for (int b = 0; b < FLIM; b += FB) {
+      T raw[FB], mk[FB], ms[FB];
+#pragma unroll
+      for (int x = 0; x < FB; ++x) {
+        const long long off = HW * (b + x < IS3 ? b + x : IS3 - 1);
+        raw[x] = mk[x] = ms[x] = T(0);
+        if (PASS != PASS_MASK_SQ) raw[x] = ldg_px<T>(p, off);
+        if (ALG == ALG_MASK_NSQECC) mk[x] = ldg_px<T>(q, off);
+        if (PASS == PASS_MASKED) ms[x] = ldg_px<T>(qs, off);
+      }
+      mqp_no_hoist();
+#pragma unroll
+      for (int x = 0; x < FB; ++x) {
+        float u = 0.f;
+        if (b + x < IS3) {
+          if (PASS == PASS_PLAIN) {
+            const T r = raw[x];
+            vmax = (double)r > vmax ? (double)r : vmax;
+            const double val = (double)r - s.meanF;
+            sumsq += val * val;
+            u = (float)val;
+          } else if (PASS == PASS_MASKED) {
+            vmax = (double)raw[x] > vmax ? (double)raw[x] : vmax;
+            mmax = (double)ms[x] > mmax ? (double)ms[x] : mmax;
+            const double val = (double)raw[x] * (double)mk[x];
+            sumsq += val * val / ((double)mk[x] > 0.0 ? (double)mk[x] : 1.0);
+            u = (float)val;
+          } else {
+            u = (float)mk[x];
+          }
         }
+        w[b + x] = u;
       }
     }
     float2 z[M];
@@ -264,14 +279,20 @@ MQP_HD MQP_FI void k3a_line(const Piv3dArgs& a, const IAGeom3& g, const IA3State
                                                                        (long long)a.W * g.g0[2]);
   const T* p = reinterpret_cast<const T*>(a.img2) + base;
   const float mg = (float)s.meanG;
+  constexpr int GB = N < 32 ? N : 32;
+  const int lo3 = g.lo[2], hi3 = g.hi[2];
 #pragma unroll
-  for (int x = 0; x < N; ++x) {
-    w[x] = 0.f;
-    if (x >= g.lo[2] && x < g.hi[2]) {
-      float v = (float)ldg_px<T>(p, HW * x);
+  for (int b = 0; b < N; b += GB) {
+    T raw[GB];
+#pragma unroll
+    for (int x = 0; x < GB; ++x) raw[x] = ldg_px<T>(p, HW * (b + x < lo3 ? lo3 : (b + x < hi3 ? b + x : hi3 - 1)));
+    mqp_no_hoist();
+#pragma unroll
+    for (int x = 0; x < GB; ++x) {
+      float v = (float)raw[x];
       if (ALG == ALG_ZNCC) v = v - mg;
       if (PASS == PASS_MASK_SQ) v = v * v;
-      w[x] = v;
+      w[b + x] = (b + x >= lo3 && b + x < hi3) ? v : 0.f;
     }
   }
   float2 z[M];
