@@ -35,7 +35,7 @@ constexpr int HUGE_THREADS = 256;
 
 // Per-block scratch slot (float2 units), sized for the pass's lags so that
 // all resident blocks' slots stay in L2:
-//   stages A-B  LG [k2][s1] (128 x P1) | GS [k2][x1] (128 x 256) | FS [k2][x1] (128 x 128)
+//   stages A-B  LG [s1][k2] (P1 x 128) | GS [k2][x1] (128 x 256) | FS [k2][x1] (128 x 128)
 //   stages C-D  LG | CC (P1 P2 floats, over the dead GS) | PL (P1 P2 doubles, after CC)
 struct HugeSlot {
   long long lg, gs, fs, cc, pl, total;
@@ -50,12 +50,17 @@ struct HugeSlot {
   }
 };
 
-// Shared memory (float2 units): the park/exchange area of stage B (64
+// Shared memory (float2 units): the area of stage B - first the G and F tiles
+// of a round's 64 columns (column stride TG / TF, odd: a warp's 32 columns fall
+// in distinct banks), then, over the G tile, the park / exchange slots (64
 // columns x 4 quarters x 64 values, element (col, q, m) at m * 256 + q * 64 +
-// col so that a warp's 32 columns fall in distinct banks), the packed column's staging (2 x 256),
-// the twiddle table (256) and reduction slots.
+// col, distinct banks again); in stage C the lag rows - the packed column's
+// staging (2 x 256), the twiddle table (256) and reduction slots.
 struct HugeSmem {
-  static constexpr int PARK = 64 * 4 * QH;
+  static constexpr int TG = NH + 1, TF = MH + 1;
+  static constexpr int FT = 64 * TG;               // F tile
+  static constexpr int PARK = FT + 64 * TF;
+  static constexpr int LS = MH + 1;                // lag row stride in stage C
   static constexpr int PACK = 2 * NH;
   static constexpr int TW = NH;
   static constexpr int RED = 32;
@@ -98,25 +103,49 @@ MQP_HD MQP_FI void huge_g_row(const Piv2dArgs& a, const IAGeom& g, float mg, int
   const T* src = reinterpret_cast<const T*>(a.img2) + ((long long)(g.g01 + t) + (long long)a.H * g.g02);
   const long long H = a.H;
   float* col = stage + t;
-  auto px = [&](int xx) {
-    float v = 0.f;
-    if (live && xx >= g.lo2 && xx < g.hi2) {
-      v = (float)ldg_px<T>(src, H * xx);
-      if (ZNCC) v -= mg;
+  // pixels load 16 at a time before any is used, at addresses clamped into the
+  // row (a dead row's into row lo1): under a condition each they cost a round
+  // trip apiece
+  constexpr int RB = 16;
+  const int lo2 = g.lo2, hi2 = g.hi2;
+  const T* lsrc = live ? src : src + (g.lo1 - t);
+  auto px = [&](int x0, float (&v)[RB]) {
+    T raw[RB];
+#pragma unroll
+    for (int k = 0; k < RB; ++k) {
+      const int x = x0 + k;
+      raw[k] = ldg_px<T>(lsrc, H * (x < lo2 ? lo2 : (x < hi2 ? x : hi2 - 1)));
     }
-    return v;
+#pragma unroll
+    for (int k = 0; k < RB; ++k) {
+      const int x = x0 + k;
+      float u = (float)raw[k];
+      if (ZNCC) u -= mg;
+      v[k] = (live && x >= lo2 && x < hi2) ? u : 0.f;
+    }
   };
-#pragma unroll 16
-  for (int x = 0; x < MH; ++x) col[x * NH] = px(x);
+#pragma unroll 2
+  for (int x = 0; x < MH; x += RB) {
+    float v[RB];
+    px(x, v);
+#pragma unroll
+    for (int k = 0; k < RB; ++k) col[(x + k) * NH] = v[k];
+  }
   float2 w[QH];
 #pragma unroll
-  for (int n = 0; n < QH; ++n) {
-    if (n % 8 == 0) mqp_no_hoist();
-    const float h0 = px(MH + 2 * n), h1 = px(MH + 2 * n + 1);
-    const float l0 = col[(2 * n) * NH], l1 = col[(2 * n + 1) * NH];
-    w[n] = make_float2(l0 + h0, l1 + h1);
-    col[(2 * n) * NH] = l0 - h0;
-    col[(2 * n + 1) * NH] = l1 - h1;
+  for (int n0 = 0; n0 < QH; n0 += RB / 2) {
+    mqp_no_hoist();
+    float v[RB];
+    px(MH + 2 * n0, v);
+#pragma unroll
+    for (int k = 0; k < RB / 2; ++k) {
+      const int n = n0 + k;
+      const float h0 = v[2 * k], h1 = v[2 * k + 1];
+      const float l0 = col[(2 * n) * NH], l1 = col[(2 * n + 1) * NH];
+      w[n] = make_float2(l0 + h0, l1 + h1);
+      col[(2 * n) * NH] = l0 - h0;
+      col[(2 * n + 1) * NH] = l1 - h1;
+    }
   }
   fft_reg<QH, false>(w);
   huge_row_bins<0>(w, GS + t, NH);
@@ -141,24 +170,29 @@ MQP_HD MQP_FI void huge_f_row(const Piv2dArgs& a, const IAGeom& g, double meanF,
   if (q < a.IS1) {
     const T* src = reinterpret_cast<const T*>(a.img1) + ((long long)(g.ir1 + q) + (long long)a.H * g.ir2);
     const long long H = a.H;
+    constexpr int RB = 32;  // pixels loaded before any is used
+    const int IS2 = a.IS2;
 #pragma unroll
-    for (int n = 0; n < QH; ++n) {
-      float v[2];
+    for (int x0 = 0; x0 < 2 * QH; x0 += RB) {
+      T raw[RB];
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int x = 2 * n + e;
-        v[e] = 0.f;
-        if (x < a.IS2) {
-          const T r = ldg_px<T>(src, H * x);
+      for (int k = 0; k < RB; ++k) raw[k] = ldg_px<T>(src, H * (x0 + k < IS2 ? x0 + k : IS2 - 1));
+      mqp_no_hoist();
+#pragma unroll
+      for (int k = 0; k < RB; ++k) {
+        float v = 0.f;
+        if (x0 + k < IS2) {
+          const T r = raw[k];
           const double val = (double)r - meanF;
           if (hh == 0) {
             vmax = (double)r > vmax ? (double)r : vmax;
             sumsq += val * val;
           }
-          v[e] = (float)val;
+          v = (float)val;
         }
+        if (k & 1) w[(x0 + k) / 2].y = v;
+        else w[(x0 + k) / 2].x = v;
       }
-      w[n] = make_float2(v[0], v[1]);
     }
     if (hh) {
 #pragma unroll
@@ -199,24 +233,31 @@ MQP_HD MQP_FI void huge_fold4(int q, Src src, const float2* tw, float2 (&y)[QH])
 // Element stride of one thread's park slots (see HugeSmem).
 constexpr int HPS = 4 * 64;
 
-// Part 1 of a column: G's quarter transformed and parked in shared memory
-// (park[m * HPS] = G^[4m + q], natural m) and F's quarter transformed into f.
-MQP_HD MQP_FI void huge_col_forward(int k2, int q, const float2* GS, const float2* FS, const float2* tw,
-                                    float2* park, float2 (&f)[QH]) {
+// Part 1 of a column: G's quarter transformed (y) and parked in shared memory
+// (park[m * HPS] = G^[4m + q], natural m), F's quarter transformed into f.
+// gc, fc: the column's 256 and 128 values.
+MQP_HD MQP_FI void huge_col_g(int q, const float2* gc, const float2* tw, float2 (&y)[QH]) {
   mqp_no_hoist();
-  {
-    float2 y[QH];
-    const float2* gc = GS + (long long)k2 * NH;
-    huge_fold4(q, [&](int j, int n) { return gc[n + QH * j]; }, tw, y);
-    fft_reg<QH, false>(y);
+  huge_fold4(q, [&](int j, int n) { return gc[n + QH * j]; }, tw, y);
+  fft_reg<QH, false>(y);
+}
+MQP_HD MQP_FI void huge_col_park(const float2 (&y)[QH], float2* park) {
 #pragma unroll
-    for (int m = 0; m < QH; ++m) park[m * HPS] = y[fpos<QH>(m)];
-  }
+  for (int m = 0; m < QH; ++m) park[m * HPS] = y[fpos<QH>(m)];
+}
+MQP_HD MQP_FI void huge_col_f(int q, const float2* fc, const float2* tw, float2 (&f)[QH]) {
   mqp_no_hoist();
-  const float2* fc = FS + (long long)k2 * MH;
   const float2 z0 = make_float2(0.f, 0.f);
   huge_fold4(q, [&](int j, int n) { return j < 2 ? fc[n + QH * j] : z0; }, tw, f);
   fft_reg<QH, false>(f);  // F^[4m + q] at f[fpos(m)]
+}
+// the packed column's spectra in natural bin order for its mirror pairs
+MQP_HD MQP_FI void huge_col_pack(int q, const float2* mine, const float2 (&f)[QH], float2* pack) {
+#pragma unroll
+  for (int m = 0; m < QH; ++m) {
+    pack[4 * m + q] = mine[m * HPS];
+    pack[NH + 4 * m + q] = f[fpos<QH>(m)];
+  }
 }
 
 // Part 2: t = conj(conj(F^) G^) for the quarter's bins, written over the
@@ -262,8 +303,8 @@ MQP_HD MQP_FI void huge_col_inverse(int q, float2* park, const float2* tw) {
 
 // Part 4 (after the quad's exchange): lags s1 = s + 64 p of the column,
 //   x[s + 64p] = sum_q W_4^{-pq} xch[q][s],   xch[q][s] = xch[s * HPS + q * 64],
-// those below P1 to LG[k2 * P1 + s1].
-MQP_HD MQP_FI void huge_col_combine(int k2, int p, int P1, const float2* xch, float2* LG) {
+// those below P1 to LG[s1 * 128 + k2] (a warp's columns are consecutive).
+MQP_HD MQP_FI void huge_col_combine(int k2, int p, int P1, const float2* xch, float2* LG) {  // LG[s1 * 128 + k2]
 #pragma unroll 4
   for (int s = 0; s < QH; ++s) {
     const int s1 = s + QH * p;
@@ -276,7 +317,7 @@ MQP_HD MQP_FI void huge_col_combine(int k2, int p, int P1, const float2* xch, fl
     else if (p == 1) v = cadd(csub(a0, a2), cmul_pi(csub(a1, a3)));
     else if (p == 2) v = csub(cadd(a0, a2), cadd(a1, a3));
     else v = cadd(csub(a0, a2), cmul_mi(csub(a1, a3)));
-    LG[(long long)k2 * P1 + s1] = v;
+    LG[(long long)s1 * MH + k2] = v;
   }
 }
 
@@ -289,15 +330,11 @@ MQP_HD MQP_FI void huge_b_part1(int r, int t, const float2* GS, const float2* FS
                                 float2* pack, float2 (&f)[QH]) {
   const int col = t % 64, q = t / 64, k2 = r * 64 + col;
   float2* mine = park + q * 64 + col;
-  huge_col_forward(k2, q, GS, FS, tw, mine, f);
-  if (k2 == 0) {
-    // the packed column's spectra in natural bin order for its mirror pairs
-#pragma unroll
-    for (int m = 0; m < QH; ++m) {
-      pack[4 * m + q] = mine[m * HPS];
-      pack[NH + 4 * m + q] = f[fpos<QH>(m)];
-    }
-  }
+  float2 y[QH];
+  huge_col_g(q, GS + (long long)k2 * NH, tw, y);
+  huge_col_park(y, mine);
+  huge_col_f(q, FS + (long long)k2 * MH, tw, f);
+  if (k2 == 0) huge_col_pack(q, mine, f, pack);
 }
 MQP_HD MQP_FI void huge_b_part2(int r, int t, const float2* tw, float2* park, const float2* pack,
                                 const float2 (&f)[QH]) {
@@ -314,11 +351,11 @@ MQP_HD MQP_FI void huge_b_part3(int r, int t, int P1, const float2* park, float2
 // ---------------------------------------------------------------------------
 // stage C: lag row s1, half hh of the complex-to-real inverse along k2
 // ---------------------------------------------------------------------------
-// As team_phase3_row with the row's spectrum X[u] = LG[u * P1 + s1].
-MQP_HD MQP_FI void huge_lag_row(int s1, int hh, int P1, int P2, const float2* LG, float* cc, float scale) {
+// As team_phase3_row with the row's spectrum X[u] = LG[s1 * ls + u].
+MQP_HD MQP_FI void huge_lag_row(int s1, int hh, int P1, int P2, const float2* LG, float* cc, float scale, int ls = MH) {
   mqp_no_hoist();
   constexpr int M = MH, Q = QH;
-  auto X = [&](int u) { return LG[(long long)u * P1 + s1]; };
+  auto X = [&](int u) { return LG[(long long)s1 * ls + u]; };
   auto tk = [](float2 A, float2 Bm, int k) {
     const float2 B = cconj(Bm);
     const float2 E = cadd(A, B);
