@@ -227,16 +227,25 @@ def run_reference(args):
 # ---------------------------------------------------------------------------
 def kernel_launches(wl, chunk3d):
     """Kernels of this library one PIV call launches (counted from the code
-    path: integral scans, the fused 2D kernel, or per 3D chunk K3a, its
-    merge, K3b, K3c and its merge)."""
+    path: integral scans and the window-sum map, the fused 2D kernel, or per 3D
+    chunk K3a, its merge, K3b, the K3c walk and its merge; FFTCC shares a
+    layer's z-spectra: one line kernel per chunk instead of K3a and its merge)."""
     scans = 0
     if wl.alg != "fft":
         per_image = 3 if wl.nd == 2 else 4  # cols, row chunks, row offsets (+ z scan)
         scans = per_image * (3 if wl.alg == "zncc" else 1)
+        if wl.alg == "nsqecc" or wl.nd == 3:
+            scans += 1
     if wl.nd == 2:
         return scans + 1
-    chunks = -(-wl.n_ia // chunk3d)
-    return scans + 5 * chunks
+    if wl.alg != "fft":
+        return scans + 5 * -(-wl.n_ia // chunk3d)
+    # chunks of whole layers, as many as half of the 1 GiB scratch budget holds spectra for
+    H, W = wl.i1.shape[:2]
+    layer = wl.vf[0] * wl.vf[1]
+    spectra = 2 * 33 * (((H + 15) // 16) | 1) * 16 * W * 8
+    layers = min(max(1, (1 << 29) // spectra), -(-chunk3d // layer))
+    return 4 * -(-wl.n_ia // min(chunk3d, layers * layer))
 
 
 def run_ours(args):

@@ -352,14 +352,117 @@ __device__ __forceinline__ int finish_search(const Piv2dArgs& a, const IAGeom& g
   return bidx;
 }
 
-// Whether an unmasked pass ends in finish_search.
+// finish_search of masked NSQECC (masked_nsqecc_ops.jl:123-142): c1(s1, s2) is
+// (F*mask)*G and c2 is mask*G^2, the window sum.  Both carry the FP32 transforms'
+// error, so the denominator may cancel where the mask covers little: it is
+// formed in FP64 as in similarity_value, and a largest value above 8 (a
+// cancelled denominator, which would scale the square root's approximation up)
+// takes the full search.
+template <int NT, typename C1, typename C2>
+__device__ __forceinline__ int finish_search_masked(const Piv2dArgs& a, const IAGeom& g, const IAScalars& sc,
+                                                    const LagRanges& R, int tid, int P1, C1 c1, C2 c2, double* red) {
+  const unsigned FULL = 0xffffffffu;
+  constexpr int NW = NT / 32;
+  const int warp = tid >> 5, lane = tid & 31;
+  if (sc.sumF2 == 0.0) return -1;  // no lag has a value above 0
+  const float sqF = sqrtf((float)sc.sumF2);
+  const bool full = !(sc.sumF2 > 1e-30 && sc.sumF2 < 1e30);
+  TopTwo t;
+  t.b1 = t.b2 = 0.f;
+  t.idx = -1;
+  const int w1 = R.hi1 - R.lo1 + 1, w2 = R.hi2 - R.lo2 + 1, total = w1 > 0 && w2 > 0 ? w1 * w2 : 0;
+  if (!full && total > 0) {
+    const int d2 = NT / w1, d1 = NT - d2 * w1;
+    int s2 = R.lo2 + tid / w1, s1 = R.lo1 + tid % w1;
+#pragma unroll 4
+    for (int q = tid; q < total; q += NT) {
+      const double S2 = c2(s1, s2);
+      const float d = sqrt_approx(fabsf((float)S2)) * sqF;
+      const double n = ((sc.sumF2 - 2.0 * c1(s1, s2)) + S2) + (double)d;
+      top_take(t, d * rcp_approx((float)n), s1 + P1 * s2);
+      s1 += d1;
+      s2 += d2;
+      if (s1 > R.hi1) {
+        s1 -= w1;
+        ++s2;
+      }
+    }
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    const float o1 = __shfl_xor_sync(FULL, t.b1, off), o2 = __shfl_xor_sync(FULL, t.b2, off);
+    const int oi = __shfl_xor_sync(FULL, t.idx, off);
+    if (o1 > t.b1) {
+      t.b2 = fmaxf(t.b1, o2);
+      t.b1 = o1;
+      t.idx = oi;
+    } else {
+      // of equal ones every lane keeps the same: they end in the full search
+      if (o1 == t.b1) t.idx = max(t.idx, oi);
+      t.b2 = fmaxf(t.b2, o1);
+    }
+  }
+  if (NT > 32) {
+    float* rf = reinterpret_cast<float*>(red);
+    if (lane == 0) {
+      rf[3 * warp] = t.b1;
+      rf[3 * warp + 1] = t.b2;
+      rf[3 * warp + 2] = __int_as_float(t.idx);
+    }
+    __syncthreads();
+    t.b1 = t.b2 = 0.f;
+    t.idx = -1;
+    for (int w = 0; w < NW; ++w) {
+      const float o1 = rf[3 * w], o2 = rf[3 * w + 1];
+      if (o1 > t.b1) {
+        t.b2 = fmaxf(t.b1, o2);
+        t.b1 = o1;
+        t.idx = __float_as_int(rf[3 * w + 2]);
+      } else {
+        t.b2 = fmaxf(t.b2, o1);
+      }
+    }
+    __syncthreads();
+  }
+  if (!full) {
+    if (!(t.b1 > 0.f)) return -1;
+    if (t.b1 <= 8.f && t.b2 < t.b1 * (1.f - PEAK_GAP)) return t.idx;
+  }
+  double best = 0.0;
+  int bidx = -1;
+#pragma unroll 1
+  for (int q = tid; q < total; q += NT) {
+    const int s1 = R.lo1 + q / w2, s2 = R.lo2 + q % w2;
+    peak_take(finish_one<ALG_MASK_NSQECC>(a, g, sc, s1, s2, c2(s1, s2), c1(s1, s2)), s1 + P1 * s2, best, bidx);
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    const double ob = __shfl_xor_sync(FULL, best, off);
+    const int oi = __shfl_xor_sync(FULL, bidx, off);
+    peak_merge(best, bidx, ob, oi);
+  }
+  if (NT > 32) {
+    if (lane == 0) {
+      red[2 * warp] = best;
+      red[2 * warp + 1] = (double)bidx;
+    }
+    __syncthreads();
+    best = red[0];
+    bidx = (int)red[1];
+    for (int w = 1; w < NW; ++w) peak_merge(best, bidx, red[2 * w], (int)red[2 * w + 1]);
+    __syncthreads();
+  }
+  return bidx;
+}
+
+// Whether a pass ends in finish_search (masked: finish_search_masked).
 MQP_HD MQP_FI bool finish_fast(const Piv2dArgs& a) { return a.SN == nullptr && a.planes == nullptr; }
 
 // refine2d_warp from the raw correlations: nine lanes evaluate the 3x3
 // neighbourhood of the peak (p1, p2) in full.
-template <int ALG, int LWN, typename CC>
-__device__ __forceinline__ void finish_refine(const Piv2dArgs& a, const IAGeom& g, const IAScalars& sc, int p1, int p2,
-                                              int lane, double scale, CC cc, const double* lw, double& r1, double& r2) {
+template <typename SIM>
+__device__ __forceinline__ void finish_refine_with(const Piv2dArgs& a, const IAGeom& g, int p1, int p2, int lane,
+                                                   SIM sim, double& r1, double& r2) {
   const unsigned FULL = 0xffffffffu;
   r1 = p1;
   r2 = p2;
@@ -367,11 +470,7 @@ __device__ __forceinline__ void finish_refine(const Piv2dArgs& a, const IAGeom& 
   const bool inside = (p1 + 1 > 1 + g.tlf1) && (p2 + 1 > 1 + g.tlf2) && (p1 + 1 < 1 + 2 * a.SM1 - g.brb1) &&
                       (p2 + 1 < 1 + 2 * a.SM2 - g.brb2);
   if (!inside) return;
-  double v = 0.0;
-  if (lane < 9) {
-    const int s1 = p1 - 1 + lane % 3, s2 = p2 - 1 + lane / 3;
-    v = finish_one<ALG, LWN>(a, g, sc, s1, s2, (double)cc(s1, s2) * scale, 0.0, lw);
-  }
+  const double v = lane < 9 ? sim(p1 - 1 + lane % 3, p2 - 1 + lane / 3) : 0.0;
   double mn = __shfl_sync(FULL, v, 0);
 #pragma unroll
   for (int k = 0; k < 9; ++k) mn = nmin(mn, __shfl_sync(FULL, v, k));
@@ -380,6 +479,14 @@ __device__ __forceinline__ void finish_refine(const Piv2dArgs& a, const IAGeom& 
   const double l[5] = {__shfl_sync(FULL, lg, 4), __shfl_sync(FULL, lg, 3), __shfl_sync(FULL, lg, 5),
                        __shfl_sync(FULL, lg, 1), __shfl_sync(FULL, lg, 7)};
   refine2d_from_logs(p1, p2, l, r1, r2);
+}
+
+template <int ALG, int LWN, typename CC>
+__device__ __forceinline__ void finish_refine(const Piv2dArgs& a, const IAGeom& g, const IAScalars& sc, int p1, int p2,
+                                              int lane, double scale, CC cc, const double* lw, double& r1, double& r2) {
+  finish_refine_with(
+      a, g, p1, p2, lane,
+      [&](int s1, int s2) { return finish_one<ALG, LWN>(a, g, sc, s1, s2, (double)cc(s1, s2) * scale, 0.0, lw); }, r1, r2);
 }
 
 #endif  // __CUDACC__

@@ -309,27 +309,50 @@ MQP_HD MQP_FI void row_process(const Piv2dArgs& a, const IAScalars& sc, int PASS
     const T* qs = PASS == PASS_MASKED ? reinterpret_cast<const T*>(a.mask_skip ? a.mask_skip : a.mask) + j.base : p;
     float w[N];
 #pragma unroll
-    for (int x = 0; x < N; ++x) {
-      w[x] = 0.f;
-      if (x < FLIM && x < j.xhi) {
-        const long long off = (long long)a.H * x;
-        if (PASS == PASS_PLAIN) {
-          const T r = ldg_px<T>(p, off);
-          vmax = (double)r > vmax ? (double)r : vmax;
-          const double val = (double)r - sc.meanF;
-          sumsq += val * val;
-          w[x] = (float)val;
-        } else if (PASS == PASS_MASKED) {
-          const T r = ldg_px<T>(p, off);
-          const T mk = ldg_px<T>(q, off);
-          const T ms = ldg_px<T>(qs, off);
-          vmax = (double)r > vmax ? (double)r : vmax;
-          mmax = (double)ms > mmax ? (double)ms : mmax;
-          const double val = (double)r * (double)mk;
-          sumsq += val * val / ((double)mk > 0.0 ? (double)mk : 1.0);
-          w[x] = (float)val;
-        } else {
-          w[x] = (float)ldg_px<T>(q, off);
+    for (int x = FLIM; x < N; ++x) w[x] = 0.f;
+    if (PASS == PASS_PLAIN) {
+      // loaded FB at a time before any is used, at addresses clamped into the
+      // row: one by one under their conditions they cost a round trip each
+      // (1501x1999 ZNCC 567 -> 529 us); whole rows do not fit beside the next
+      // row's prefetch (737), nor do the masked passes' three images (390 -> 482)
+      constexpr int FB = 16;
+#pragma unroll
+      for (int b = 0; b < FLIM; b += FB) {
+        T raw[FB];
+#pragma unroll
+        for (int x = 0; x < FB; ++x) raw[x] = ldg_px<T>(p, (long long)a.H * (b + x < j.xhi ? b + x : j.xhi - 1));
+        mqp_no_hoist();
+#pragma unroll
+        for (int x = 0; x < FB; ++x) {
+          float u = 0.f;
+          if (b + x < j.xhi) {
+            const T r = raw[x];
+            vmax = (double)r > vmax ? (double)r : vmax;
+            const double val = (double)r - sc.meanF;
+            sumsq += val * val;
+            u = (float)val;
+          }
+          w[b + x] = u;
+        }
+      }
+    } else {
+#pragma unroll
+      for (int x = 0; x < FLIM; ++x) {
+        w[x] = 0.f;
+        if (x < j.xhi) {
+          const long long off = (long long)a.H * x;
+          if (PASS == PASS_MASKED) {
+            const T r = ldg_px<T>(p, off);
+            const T mk = ldg_px<T>(q, off);
+            const T ms = ldg_px<T>(qs, off);
+            vmax = (double)r > vmax ? (double)r : vmax;
+            mmax = (double)ms > mmax ? (double)ms : mmax;
+            const double val = (double)r * (double)mk;
+            sumsq += val * val / ((double)mk > 0.0 ? (double)mk : 1.0);
+            w[x] = (float)val;
+          } else {
+            w[x] = (float)ldg_px<T>(q, off);
+          }
         }
       }
     }

@@ -115,6 +115,26 @@ __device__ __forceinline__ void piv2d_big_ia(const Piv2dArgs& a, long long ia, f
   R.hi2 = 2 * a.SM2 - g.brb2;
   R.shi1 = 2 * a.SM1 - 1 - g.brb1;
   R.shi2 = 2 * a.SM2 - 1 - g.brb2;
+  if constexpr (MASKED) {
+    if (finish_fast(a)) {
+      auto c1 = [&](int s1, int s2) { return (double)c1buf[s1 * P2 + s2]; };
+      auto c2 = [&](int s1, int s2) { return plane[s1 * P2 + s2]; };
+      const int bidx = finish_search_masked<BIG_THREADS>(a, g, sc, R, t, P1, c1, c2, red);
+      if (warp == 0) {
+        double r1 = -1.0, r2 = -1.0;  // no peak: 1-based (0, 0), displacement -(SM+1)
+        if (bidx >= 0)
+          finish_refine_with(
+              a, g, bidx % P1, bidx / P1, lane,
+              [&](int s1, int s2) { return finish_one<ALG>(a, g, sc, s1, s2, c2(s1, s2), c1(s1, s2)); }, r1, r2);
+        if (lane == 0) {
+          a.VF[2 * vfo + 0] = r1 - a.SM1 + d1;
+          a.VF[2 * vfo + 1] = r2 - a.SM2 + d2;
+        }
+      }
+      __syncthreads();
+      return;
+    }
+  }
   if constexpr (!MASKED) {
     if (finish_fast(a)) {
       auto cc = [&](int s1, int s2) { return (float)plane[s1 * P2 + s2]; };  // exact: FP32 times a power of two

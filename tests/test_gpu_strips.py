@@ -64,3 +64,23 @@ def test_ties_skips_and_scales(alg, gpu):
     _both(tile, tile, False, **kw)
     for s in (1e-18, 1e17):
         _both(noise * np.float32(s), noise * np.float32(s), False, **kw)
+
+
+@pytest.mark.parametrize("IS,SM,st", [(16, 8, 8), (32, 16, 13), (24, 11, 12), (64, 32, 32), (48, 20, 21)])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_masked_walk_equals_full_search(IS, SM, st, dtype, gpu):
+    """Masked NSQECC without SN (the approximate walk) against the same pass
+    with SN (every lag in full), with areas the mask covers fully, partly, by a
+    few pixels and not at all."""
+    import torch
+    i1, i2, _ = synth.pair_2d_shift(shape=(203, 177), shift=(2.6, -3.3), seed_stream=45, dtype=dtype)
+    g = np.random.default_rng(9)
+    mask = np.zeros(i1.shape, dtype=dtype)
+    mask[30:140, 20:120] = 1
+    mask[::37, ::29] = 1  # lone pixels
+    mask[60:80, 60:80] = g.uniform(0, 1, (20, 20))
+    d = [torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in (i1, i2, mask)]
+    kw = dict(interSize=(IS, IS), searchMargin=(SM, SM), step=(st, st))
+    walk = PIV(*d, setPIVParameters(**kw))[0].cpu().numpy()
+    full = PIV(*d, setPIVParameters(computeSN=True, **kw))[0].cpu().numpy()
+    assert np.array_equal(walk, full, equal_nan=True)
