@@ -21,9 +21,9 @@
 // eight.  Each value goes through the same operations in the same order as
 // there: the fields are the same bit for bit.
 //
-// Bound by instruction issue and supply: 9.5k warp instructions per IA (15.3k
-// before), issue active 45 %, stalls led by no_instruction (1.25 warps per
-// issue) and the barrier after the rows (1.07).  Measured on B200 (kernel,
+// Bound by instruction issue and supply (ncu, 1024^2 NSQECC step 8): 11.6k warp
+// instructions per IA (15.3k before), issue active 54 %, stalls led by
+// no_instruction (0.95 warps per issue) and wait (0.93).  Measured on B200 (kernel,
 // one warp per IA -> strips): 2048^2 NSQECC step 8 2113 -> 1202 us, FFTCC 1270 ->
 // 1023; 1024x1280 NSQECC step 16 199 -> 93; 2048^2 NSQECC step 16 with SN 589 ->
 // 354; 256^2 FFTCC Float64 step 16 35 -> 17.
