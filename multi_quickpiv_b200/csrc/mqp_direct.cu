@@ -382,7 +382,7 @@ __global__ void __launch_bounds__(D3T_MAXT) direct3d_tiled_kernel(Piv3dArgs a, i
 
 // grid: resident blocks of `kern` with `smem` bytes, at most enough for n warps' work
 cudaError_t grid_for(const void* kern, size_t smem, long long n, long long& blocks, std::string& err) {
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_dyn_smem(kern, smem);
   if (e != cudaSuccess) {
     err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e);
     return e;
@@ -442,7 +442,7 @@ cudaError_t d3t_launch(const Piv3dArgs& a, cudaStream_t s, std::string& err) {
   const int tasks = (2 * a.SM[0] + 1) * (2 * a.SM[2] + 1);
   const int nt = std::min(D3T_MAXT, (tasks + 31) / 32 * 32);
   const void* kern = (const void*)direct3d_tiled_kernel<ALG, T, IS2, P2>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_dyn_smem(kern, smem);
   int dev = 0, per_sm = 0;
   if (e == cudaSuccess) e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nt, smem);

@@ -59,6 +59,18 @@ cudaError_t launch_piv2d(const Piv2dArgs& a, int alg, cudaStream_t s, std::strin
 
 int device_sm_count(int device);
 
+// Lets `kern` launch with `smem` bytes of dynamic shared memory.  The limit
+// belongs to the function, not to the launch: threads that each wrote their
+// own launch's size could leave a launch under another's smaller limit
+// (cudaErrorInvalidValue).  So every caller writes the same value, a block's
+// 227 KB less the few bytes of static shared memory that some kernels have.
+constexpr size_t DYN_SMEM_LIMIT = 227 * 1024 - 16;
+template <typename K>
+cudaError_t allow_dyn_smem(K kern, size_t smem) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)(smem > DYN_SMEM_LIMIT ? smem : DYN_SMEM_LIMIT));
+}
+
 // the warp kernels' launches per FFT length (mqp_piv2d_w*.cu, mqp_piv2d_b*.cu)
 struct Piv2dBatch;
 cudaError_t launch_piv2d_w64(const Piv2dArgs& a, int alg, bool prune, cudaStream_t s, std::string& err);

@@ -251,7 +251,7 @@ cudaError_t big_launch(const Piv2dArgs* single, const Piv2dBatch* batch, cudaStr
   const size_t smem = (size_t)wsz * sizeof(float2);
   const void* kern = single ? (const void*)piv2d_big_kernel<FPRUNE, ALG, T>
                             : (const void*)piv2d_big_batch_kernel<FPRUNE, ALG, T>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_dyn_smem(kern, smem);
   if (e != cudaSuccess) {
     err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e);
     return e;

@@ -258,7 +258,7 @@ template <int ALG, typename T>
 cudaError_t launch_huge_t(const Piv2dArgs& a, cudaStream_t s, std::string& err) {
   const size_t smem = (size_t)HugeSmem::TOTAL * sizeof(float2);
   auto kern = piv2d_huge_kernel<ALG, T>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_dyn_smem(kern, smem);
   if (e != cudaSuccess) {
     err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e);
     return e;

@@ -628,7 +628,7 @@ StripCfg strip_cfg(const Piv2dArgs& a, int n, int wpi) {
 template <int ALG, typename T, bool SN>
 cudaError_t strip_launch(const Piv2dArgs& a, const StripCfg& c, cudaStream_t s, std::string& err) {
   auto kern = strip_kernel<ALG, T, SN>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.bytes);
+  cudaError_t e = allow_dyn_smem(kern, c.bytes);
   if (e != cudaSuccess) {
     err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e);
     return e;

@@ -317,7 +317,7 @@ struct TeamCfg<32> {
 template <typename K>
 cudaError_t grid_for(K kern, int threads, size_t smem, long long work, long long per_block, long long& blocks,
                      std::string& err) {
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_dyn_smem(kern, smem);
   if (e != cudaSuccess) {
     err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e);
     return e;

@@ -439,7 +439,7 @@ static cudaError_t launch_t(const Piv2dArgs& a, cudaStream_t s, std::string& err
   CUtensorMap tmap;
   memset(&tmap, 0, sizeof(tmap));
   if (tm) tmap = *tm;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_dyn_smem(kern, smem);
   if (e != cudaSuccess) {
     err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e);
     return e;
@@ -516,7 +516,7 @@ template <int N, bool FPRUNE, int ALG, typename T, int WARPS, int MINB, bool LW 
 static cudaError_t launch_batch_t(const Piv2dBatch& b, cudaStream_t s, std::string& err) {
   const size_t smem = ((size_t)WARPS * b.wf2 + N) * sizeof(float2);
   auto kern = piv2d_batch_kernel<N, FPRUNE, ALG, T, WARPS, MINB, LW>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_dyn_smem(kern, smem);
   if (e != cudaSuccess) {
     err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e);
     return e;

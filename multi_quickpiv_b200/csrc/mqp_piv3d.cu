@@ -569,7 +569,7 @@ cudaError_t run_chunks(Piv3dArgs a, long long chunk, cudaStream_t s, std::string
   if constexpr (CAN_SHARE) {
     if (shared) k3b = k3b_kernel<N, FPRUNE, true>;
   }
-  cudaError_t e = cudaFuncSetAttribute(k3b, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_dyn_smem(k3b, smem);
   if (e != cudaSuccess) {
     err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e);
     return e;
