@@ -137,11 +137,13 @@ __device__ __forceinline__ void piv2d_big_ia(const Piv2dArgs& a, long long ia, f
   }
   if constexpr (!MASKED) {
     if (finish_fast(a)) {
-      auto cc = [&](int s1, int s2) { return (float)plane[s1 * P2 + s2]; };  // exact: FP32 times a power of two
-      const int bidx = finish_search<ALG, BIG_THREADS, 0>(a, g, sc, R, t, P1, 1.0, cc, nullptr, red);
+      // the transforms' FP32 value: the plane's, times a power of two, may lie below FP32's normal range
+      const double scale = cc_scale<NB>();
+      auto cc = [&](int s1, int s2) { return (float)(plane[s1 * P2 + s2] * (1.0 / cc_scale<NB>())); };
+      const int bidx = finish_search<ALG, BIG_THREADS, 0>(a, g, sc, R, t, P1, scale, cc, nullptr, red);
       if (warp == 0) {
         double r1 = -1.0, r2 = -1.0;  // no peak: 1-based (0, 0), displacement -(SM+1)
-        if (bidx >= 0) finish_refine<ALG, 0>(a, g, sc, bidx % P1, bidx / P1, lane, 1.0, cc, nullptr, r1, r2);
+        if (bidx >= 0) finish_refine<ALG, 0>(a, g, sc, bidx % P1, bidx / P1, lane, scale, cc, nullptr, r1, r2);
         if (lane == 0) {
           a.VF[2 * vfo + 0] = r1 - a.SM1 + d1;
           a.VF[2 * vfo + 1] = r2 - a.SM2 + d2;

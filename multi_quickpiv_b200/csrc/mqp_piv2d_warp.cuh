@@ -302,11 +302,12 @@ __device__ __forceinline__ void piv2d_ia(const Piv2dArgs& a, long long ia, float
   }
   if constexpr (!MASKED) {
     if (finish_fast(a)) {
-      auto cc = [&](int s1, int s2) { return (float)plane[s1 * P2 + s2]; };  // exact: FP32 times a power of two
-      const int bidx = finish_search<ALG, 32, LW ? N : 0>(a, g, sc, R, lane, P1, 1.0, cc, lw, nullptr);
+      // the transforms' FP32 value: the plane's, times a power of two, may lie below FP32's normal range
+      auto cc = [&](int s1, int s2) { return (float)(plane[s1 * P2 + s2] * (1.0 / cc_scale<N>())); };
+      const int bidx = finish_search<ALG, 32, LW ? N : 0>(a, g, sc, R, lane, P1, scale, cc, lw, nullptr);
       double r1 = -1.0, r2 = -1.0;  // no peak: 1-based (0, 0), displacement -(SM+1)
       if (bidx >= 0)
-        finish_refine<ALG, LW ? N : 0>(a, g, sc, bidx % P1, bidx / P1, lane, 1.0, cc, lw, r1, r2);
+        finish_refine<ALG, LW ? N : 0>(a, g, sc, bidx % P1, bidx / P1, lane, scale, cc, lw, r1, r2);
       __syncwarp();
       if (LW) stage_next();
       if (lane == 0) {

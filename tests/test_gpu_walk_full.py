@@ -1,0 +1,40 @@
+"""Passes without SN, which search the peak among FP32 approximations, against
+the same passes with SN, which evaluate every lag in full: the same fields bit
+for bit."""
+import numpy as np
+import pytest
+
+from multi_quickpiv_b200 import PIV, setPIVParameters
+
+pytestmark = pytest.mark.gpu
+
+
+def _walk_equals_full(i1, i2, mask=None, **kw):
+    import torch
+    d = [torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in (i1, i2) + (() if mask is None else (mask,))]
+    walk = PIV(*d, setPIVParameters(**kw))[0].cpu().numpy()
+    full = PIV(*d, setPIVParameters(computeSN=True, **kw))[0].cpu().numpy()
+    assert np.array_equal(walk, full, equal_nan=True), int((walk != full).sum())
+    return walk
+
+
+def _spots(shape, g, n):
+    a, b = np.zeros(shape), np.zeros(shape)
+    at, peak = g.integers(0, np.array(shape), (n, len(shape))), g.uniform(0.5, 1, n)
+    np.add.at(a, tuple(at.T), peak)
+    np.add.at(b, tuple(np.minimum(at + 2, np.array(shape) - 1).T), peak)
+    return a, b
+
+
+# FFT lengths 32, 64 (one warp per area: steps above the window, more than 36 lag rows) and 128, 64 in strips
+@pytest.mark.parametrize("IS,SM,st", [((16, 16), (8, 8), (5, 9)), ((32, 32), (16, 16), (40, 40)),
+                                      ((12, 30), (19, 2), (12, 30)), ((64, 64), (32, 32), (32, 32)),
+                                      ((32, 32), (16, 16), (8, 8))])
+@pytest.mark.parametrize("scale", [1e-19, 1e-20, 2e-21])
+def test_faint_images(IS, SM, st, scale, gpu):
+    """Pixels whose correlation lies at the low end of FP32's range: the
+    similarities are those of the transforms' own FP32 values."""
+    a, b = _spots((437, 391), np.random.default_rng(7), 3400)
+    i1, i2 = (a * scale).astype(np.float32), (b * scale).astype(np.float32)
+    VF = _walk_equals_full(i1, i2, corr_alg="nsqecc", interSize=IS, searchMargin=SM, step=st)
+    assert np.isfinite(VF).mean() > 0.5
