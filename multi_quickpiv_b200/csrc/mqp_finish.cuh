@@ -13,14 +13,17 @@
 //
 // NSQECC, v = d / (d + n) with d = sqrt(S2) sqrt(F2) and n = F2 + S2 - 2c
 // (nsqecc_ops.jl:1-25): d is formed from the same FP32 square roots as in
-// similarity_value.  n >= 0 up to the correlation's rounding (Cauchy), so
-// F2 + S2 <= d + n + 4d and the terms of d + n add up to at most five times
-// their sum; with three FP32 roundings each, the sum is within 9e-7 of exact,
-// the approximate reciprocal and the product add 2e-7, and the full value's
-// own FP32 steps 2e-7.  ZNCC, v = c / (sqrt(SG) sqrt(F2)) (zncc_ops.jl:29-50):
-// SG is formed in FP64 as in similarity_value, its approximate inverse square
-// root and the product are within 4e-7, the full value within 2e-7; the
-// factor 1 / sqrt(F2) is common to the box and left out.
+// similarity_value.  By Cauchy, d + n = F2 + S2 + d - 2c is at least (F2 + S2) / 2
+// - but c is the FP32 transforms' correlation, whose error grows with the whole
+// search window: beside pixels some 10^6 times brighter the sum may cancel.  A
+// lag whose sum falls below a quarter of F2 + S2 sends the area to the full
+// search (nsqecc_walk).  Above that the terms of the sum add up to at most
+// seven times it; F2 and S2 in FP32 and the three FP32 additions leave it
+// within 8e-7 of exact, the approximate reciprocal and the product add 2e-7,
+// and the full value's own FP32 steps 2e-7.  ZNCC, v = c / (sqrt(SG) sqrt(F2))
+// (zncc_ops.jl:29-50): SG is formed in FP64 as in similarity_value, its
+// approximate inverse square root and the product are within 4e-7, the full
+// value within 2e-7; the factor 1 / sqrt(F2) is common to the box and left out.
 #pragma once
 
 #include "mqp_piv2d.cuh"
@@ -72,9 +75,7 @@ MQP_HD MQP_FI void first_take(TopTwo& t, float v, int idx) {
   }
 }
 
-#if defined(__CUDACC__)
-
-__device__ __forceinline__ float rcp_approx(float x) {
+MQP_HD MQP_FI float rcp_approx(float x) {
 #if defined(__CUDA_ARCH__)
   float r;
   asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -83,6 +84,37 @@ __device__ __forceinline__ float rcp_approx(float x) {
   return 1.f / x;
 #endif
 }
+MQP_HD MQP_FI float sqrt_approx(float x) {
+#if defined(__CUDA_ARCH__)
+  float r;
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+#else
+  return sqrtf(x);
+#endif
+}
+MQP_HD MQP_FI int sign_word(float x) {  // negative when x's sign bit is set
+#if defined(__CUDA_ARCH__)
+  return __float_as_int(x);
+#else
+  return signbit(x) ? -1 : 0;
+#endif
+}
+
+// The walk's similarity of one lag from its raw correlation c; open turns
+// negative (and stays so over the lags) where the approximation is not within
+// the bounds above.  NSQECC: S2 and its root, m2 = -2 times the correlation's
+// scale.
+MQP_HD MQP_FI float nsqecc_walk(float S2, float root, float c, float m2, float F2, float sqF, int& open) {
+  const float d = root * sqF, t = F2 + S2, den = fmaf(m2, c, t) + d;
+  open |= sign_word(fmaf(-0.25f, t, den));
+  return d * rcp_approx(den);
+}
+// A lane that met an open lag: two values no other lane's can exceed, so that
+// the search does not end on one lag.
+MQP_HD MQP_FI void top_open(TopTwo& t) { t.b1 = t.b2 = INFINITY; }
+
+#if defined(__CUDACC__)
 
 // The lags of the box that the map does not hold (rows past e1, then columns
 // past e2), over the lanes.
@@ -95,16 +127,6 @@ __device__ __forceinline__ void unmapped_lags(const LagRanges& R, int e1, int e2
     if (q < nr) take(R.hi1 - q / w2, R.lo2 + q % w2);
     else take(R.lo1 + (q - nr) % h1, R.hi2 - (q - nr) / h1);
   }
-}
-
-__device__ __forceinline__ float sqrt_approx(float x) {
-#if defined(__CUDA_ARCH__)
-  float r;
-  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-#else
-  return sqrtf(x);
-#endif
 }
 
 // Lag box walk of NT threads (one warp, or a block whose every thread calls
@@ -137,6 +159,7 @@ __device__ __forceinline__ int finish_search(const Piv2dArgs& a, const IAGeom& g
   // lag q of the walk: s1 = lo1 + q % w1, s2 = lo2 + q / w1, so that a warp
   // reads runs of consecutive rows
   const int w1 = e1 - R.lo1 + 1, total = w1 > 0 && e2 >= R.lo2 ? w1 * (e2 - R.lo2 + 1) : 0;
+  int open = 0;
   if (!full && total > 0) {
     const int d2 = NT / w1, d1 = NT - d2 * w1;
     int s2 = R.lo2 + tid / w1, s1 = R.lo1 + tid % w1;
@@ -199,10 +222,7 @@ __device__ __forceinline__ int finish_search(const Piv2dArgs& a, const IAGeom& g
           }
         }
       };
-      auto nsqecc = [&](float s, float q, float c) {
-        const float d = q * sqF;
-        return d * rcp_approx(fmaf(m2, c, F2 + s) + d);
-      };
+      auto nsqecc = [&](float s, float q, float c) { return nsqecc_walk(s, q, c, m2, F2, sqF, open); };
       auto zncc = [&](double S2, double S1, double n, float c) {
         const double SG = S2 - 2.0 * sc.meanG * S1 + n * sc.meanG * sc.meanG;
         return c * fscale * rsqrtf((float)(SG > 0.0 ? SG : 0.0));
@@ -268,6 +288,7 @@ __device__ __forceinline__ int finish_search(const Piv2dArgs& a, const IAGeom& g
       top_take(t, ALG == ALG_ZNCC ? v * sqF : v, s1 + P1 * s2);  // on the walk's scale
     }
   }
+  if (open < 0) top_open(t);
   // the largest value of the box, and what comes within the gap of it
   float* redf = reinterpret_cast<float*>(red);
   const int warp = tid >> 5, lane = tid & 31;

@@ -366,6 +366,7 @@ __global__ void __launch_bounds__(K3C_THREADS, N <= 64 ? 2 : 1) k3c_walk_kernel(
   TopTwo t;
   t.b1 = t.b2 = 0.f;
   t.idx = -1;
+  int open = 0;
 #pragma unroll 1
   for (int q = q0 + threadIdx.x; q < q1; q += blockDim.x) {
     const int s1 = q % P1, s2 = q / P1;
@@ -411,8 +412,7 @@ __global__ void __launch_bounds__(K3C_THREADS, N <= 64 ? 2 : 1) k3c_walk_kernel(
             if (ALG == ALG_FFTCC) {
               first_take(t, c, idx);
             } else if (ALG == ALG_NSQECC) {
-              const float d = m[k].y * sqF;
-              top_take(t, d * rcp_approx(fmaf(m2, c, F2 + m[k].x) + d), idx);
+              top_take(t, nsqecc_walk(m[k].x, m[k].y, c, m2, F2, sqF, open), idx);
             } else {
               int z0, z1;
               lag_window(s3, a.IS[2], g.g0[2], g.lo[2], g.hi[2], z0, z1);
@@ -440,6 +440,7 @@ __global__ void __launch_bounds__(K3C_THREADS, N <= 64 ? 2 : 1) k3c_walk_kernel(
       }
     }
   }
+  if (open < 0) top_open(t);
   // the block's two largest
   __shared__ TopPart3 red[K3C_THREADS / 32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

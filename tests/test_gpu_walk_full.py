@@ -38,3 +38,17 @@ def test_faint_images(IS, SM, st, scale, gpu):
     i1, i2 = (a * scale).astype(np.float32), (b * scale).astype(np.float32)
     VF = _walk_equals_full(i1, i2, corr_alg="nsqecc", interSize=IS, searchMargin=SM, step=st)
     assert np.isfinite(VF).mean() > 0.5
+
+
+@pytest.mark.parametrize("shape,IS,SM,st,seed", [((2048, 2048), 64, 96, 15, 0), ((2048, 2048), 32, 48, 7, 0),
+                                                 ((256, 256, 192), 16, 20, 8, 0), ((256, 256, 192), 16, 20, 8, 1)])
+def test_bright_pixels_beside_dark_windows(shape, IS, SM, st, seed, gpu):
+    """Pixels 1e9 times brighter than the rest: the transforms' error, which
+    grows with the whole search window, cancels NSQECC denominators of the
+    windows that hold none of them."""
+    g, nd = np.random.default_rng(seed), len(shape)
+    a = g.uniform(0.5, 1.5, shape)
+    b = a.copy()
+    b[tuple(g.integers(0, np.array(shape), (int(np.prod(shape)) // (1500 if nd == 2 else 20000), nd)).T)] = 1e9
+    _walk_equals_full(a.astype(np.float32), b.astype(np.float32), corr_alg="nsqecc", interSize=(IS,) * nd,
+                      searchMargin=(SM,) * nd, step=(st,) * nd)
