@@ -110,6 +110,15 @@ MQP_HD MQP_FI float nsqecc_walk(float S2, float root, float c, float m2, float F
   open |= sign_word(fmaf(-0.25f, t, den));
   return d * rcp_approx(den);
 }
+// Masked NSQECC, c1 = (F*mask)*G and S2 = mask*G^2; most keeps the largest
+// magnitude, above 8 = open.
+MQP_HD MQP_FI float masked_walk(double S2, double c1, double sumF2, float sqF, float& most) {
+  const float d = sqrt_approx(fabsf((float)S2)) * sqF;
+  const double n = ((sumF2 - 2.0 * c1) + S2) + (double)d;
+  const float v = d * rcp_approx((float)n);
+  most = fmaxf(most, fabsf(v));
+  return v;
+}
 // A lane that met an open lag: two values no other lane's can exceed, so that
 // the search does not end on one lag.
 MQP_HD MQP_FI void top_open(TopTwo& t) { t.b1 = t.b2 = INFINITY; }
@@ -376,9 +385,9 @@ __device__ __forceinline__ int finish_search(const Piv2dArgs& a, const IAGeom& g
 // finish_search of masked NSQECC (masked_nsqecc_ops.jl:123-142): c1(s1, s2) is
 // (F*mask)*G and c2 is mask*G^2, the window sum.  Both carry the FP32 transforms'
 // error, so the denominator may cancel where the mask covers little: it is
-// formed in FP64 as in similarity_value, and a largest value above 8 (a
-// cancelled denominator, which would scale the square root's approximation up)
-// takes the full search.
+// formed in FP64 as in similarity_value, and a value above 8 of either sign (a
+// cancelled denominator, which scales the square root's approximation up and
+// may come out of it with the other sign) takes the full search.
 template <int NT, typename C1, typename C2>
 __device__ __forceinline__ int finish_search_masked(const Piv2dArgs& a, const IAGeom& g, const IAScalars& sc,
                                                     const LagRanges& R, int tid, int P1, C1 c1, C2 c2, double* red) {
@@ -392,15 +401,13 @@ __device__ __forceinline__ int finish_search_masked(const Piv2dArgs& a, const IA
   t.b1 = t.b2 = 0.f;
   t.idx = -1;
   const int w1 = R.hi1 - R.lo1 + 1, w2 = R.hi2 - R.lo2 + 1, total = w1 > 0 && w2 > 0 ? w1 * w2 : 0;
+  float most = 0.f;
   if (!full && total > 0) {
     const int d2 = NT / w1, d1 = NT - d2 * w1;
     int s2 = R.lo2 + tid / w1, s1 = R.lo1 + tid % w1;
 #pragma unroll 4
     for (int q = tid; q < total; q += NT) {
-      const double S2 = c2(s1, s2);
-      const float d = sqrt_approx(fabsf((float)S2)) * sqF;
-      const double n = ((sc.sumF2 - 2.0 * c1(s1, s2)) + S2) + (double)d;
-      top_take(t, d * rcp_approx((float)n), s1 + P1 * s2);
+      top_take(t, masked_walk(c2(s1, s2), c1(s1, s2), sc.sumF2, sqF, most), s1 + P1 * s2);
       s1 += d1;
       s2 += d2;
       if (s1 > R.hi1) {
@@ -409,6 +416,7 @@ __device__ __forceinline__ int finish_search_masked(const Piv2dArgs& a, const IA
       }
     }
   }
+  if (most > 8.f) top_open(t);
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) {
     const float o1 = __shfl_xor_sync(FULL, t.b1, off), o2 = __shfl_xor_sync(FULL, t.b2, off);
@@ -447,7 +455,7 @@ __device__ __forceinline__ int finish_search_masked(const Piv2dArgs& a, const IA
   }
   if (!full) {
     if (!(t.b1 > 0.f)) return -1;
-    if (t.b1 <= 8.f && t.b2 < t.b1 * (1.f - PEAK_GAP)) return t.idx;
+    if (t.b2 < t.b1 * (1.f - PEAK_GAP)) return t.idx;
   }
   double best = 0.0;
   int bidx = -1;

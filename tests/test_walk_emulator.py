@@ -51,3 +51,27 @@ def test_nsqecc_approximation(emu, F2):
         S2b, cb = S2.copy(), c.copy()
         S2b[at], cb[at] = s2, bad
         assert _nsqecc(emu, S2b, cb, F2)[0] == expect
+
+
+@pytest.mark.parametrize("F2", [1e-29, 3.7, 9e29])
+def test_masked_approximation(emu, F2):
+    """Masked lags within the bound keep the full value; a cancelled denominator
+    opens the area also where the approximate root leaves it negative."""
+    g = np.random.default_rng(4)
+    S2 = F2 * 10 ** g.uniform(-6, 6, 4000) * np.where(g.uniform(size=4000) < 0.1, -1, 1)  # the transforms' error has no sign
+    d = np.sqrt(np.abs(S2) * F2)
+    share = g.uniform(0.15, 3, 4000) * np.where(g.uniform(size=4000) < 0.3, -1, 1)  # denominator / d
+    c1 = (F2 + S2 + d - share * d) / 2
+    emu.mqp_walk_masked.restype = C.c_float
+
+    def run(c1):
+        walk, full = np.zeros(4000), np.zeros(4000)
+        return emu.mqp_walk_masked(4000, _p(S2), _p(c1), C.c_double(F2), _p(walk), _p(full)), walk, full
+
+    most, walk, full = run(c1)
+    assert most <= 8
+    assert np.max(np.abs(walk / full - 1)) < 4 * EPS32  # the same denominator; reciprocal and product against a quotient
+    for part in (0.1, 1e-3, 1e-6, -1e-6, -1e-3, -0.1):
+        cb, at = c1.copy(), g.integers(0, 4000)
+        cb[at] = (F2 + S2[at] + d[at] - part * d[at]) / 2
+        assert run(cb)[0] > 8
