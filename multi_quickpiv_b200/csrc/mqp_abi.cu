@@ -119,13 +119,12 @@ static int integrals_2d(mqp_ctx* ctx, const Problem& pb, const void* d1, const v
   return MQP_OK;
 }
 
-// The window-sum map of a 2D pass that takes one (ctx buffer), after the
-// integral columns of image columns [0, x1): map columns [*m0, ...) as far as
-// those go; *m0 moves on.
-static int window_map_2d(mqp_ctx* ctx, const Problem& pb, bool SN, bool pred, cudaStream_t s, int x1, int* m0) {
-  if (!mqp::piv2d_takes_map(pb.IS[0], pb.IS[1], pb.SM[0], pb.SM[1], pb.alg, SN, pred)) return MQP_OK;
-  const int H = (int)pb.dims[0], W = (int)pb.dims[1];
-  auto layout = [&](void* base) { return mqp::window_map(H, W, pb.IS[0], pb.IS[1], pb.SM[0], pb.SM[1], pb.alg, SN, base); };
+// The window-sum map of a 2D pass that takes one (ctx buffer), bound to `a`
+// (the whole pass), after the integral columns of image columns [0, x1): map
+// columns [*m0, ...) as far as those go; *m0 moves on.
+static int window_map_2d(mqp_ctx* ctx, mqp::Piv2dArgs& a, int alg, cudaStream_t s, int x1, int* m0) {
+  if (!mqp::piv2d_takes_map(a, alg)) return MQP_OK;
+  auto layout = [&](void* base) { return mqp::window_map(a.H, a.W, a.IS1, a.IS2, a.SM1, a.SM2, alg, a.SN != nullptr, base); };
   cudaError_t e = ctx->wmap.ensure(layout(nullptr).bytes);
   if (e == cudaErrorMemoryAllocation) {  // the kernels read the integral images instead
     cudaGetLastError();
@@ -133,12 +132,15 @@ static int window_map_2d(mqp_ctx* ctx, const Problem& pb, bool SN, bool pred, cu
   }
   if (e != cudaSuccess) return cuda_fail(ctx, e, "window-sum map");
   const mqp::WindowMap m = layout(ctx->wmap.ptr);
-  const int m1 = x1 == W ? m.cols : std::min(m.cols, std::max(*m0, x1 - pb.IS[1] + pb.SM[1] + 1));
+  const int m1 = x1 == a.W ? m.cols : std::min(m.cols, std::max(*m0, x1 - a.IS2 + a.SM2 + 1));
   ProfileScope ps(ctx, s, 0, 0);
-  if (m1 > *m0 && (e = mqp::launch_window_map((const double*)ctx->IIg2.ptr, (const double*)ctx->IIg.ptr, H, W, pb.IS[0],
-                                              pb.IS[1], pb.SM[0], pb.SM[1], m, *m0, m1, s)) != cudaSuccess)
+  if (m1 > *m0 && (e = mqp::launch_window_map(a.IIg2, a.IIg, a.H, a.W, a.IS1, a.IS2, a.SM1, a.SM2, m, *m0, m1, s)) != cudaSuccess)
     return cuda_fail(ctx, e, "window-sum map");
   *m0 = m1;
+  a.ws = m.ws;
+  a.wd = m.wd;
+  a.wz = m.wz;
+  a.ldw = m.ldw;
   return MQP_OK;
 }
 
@@ -159,16 +161,6 @@ static mqp::Piv2dArgs args_2d(mqp_ctx* ctx, const Problem& pb, const mqp_params*
   if (pb.alg == mqp::ALG_ZNCC) {
     a.IIg = (const double*)ctx->IIg.ptr;
     a.II1 = (const double*)ctx->II1.ptr;
-  }
-  if (mqp::piv2d_takes_map(pb.IS[0], pb.IS[1], pb.SM[0], pb.SM[1], pb.alg, dSN != nullptr, dpred != nullptr)) {
-    const mqp::WindowMap m = mqp::window_map((int)pb.dims[0], (int)pb.dims[1], pb.IS[0], pb.IS[1], pb.SM[0], pb.SM[1],
-                                             pb.alg, dSN != nullptr, ctx->wmap.ptr);
-    if (ctx->wmap.bytes >= m.bytes) {
-      a.ws = m.ws;
-      a.wd = m.wd;
-      a.wz = m.wz;
-      a.ldw = m.ldw;
-    }
   }
   a.pred = dpred;
   a.VF = dVF;
@@ -216,9 +208,9 @@ int run_pass_2d(mqp_ctx* ctx, const Problem& pb, const mqp_params* p, const void
   if (pb.IS[0] > H || pb.IS[1] > W) return MQP_OK;  // empty vector field
   int rc = integrals_2d(ctx, pb, d1, d2, dtype, s, 0, W);
   if (rc != MQP_OK) return rc;
-  int m0 = 0;
-  if ((rc = window_map_2d(ctx, pb, dSN != nullptr, dpred != nullptr, s, W, &m0)) != MQP_OK) return rc;
   mqp::Piv2dArgs a = args_2d(ctx, pb, p, d1, d2, dmask, dskip, dtype, dVF, dSN, dpred, dplanes, ia_begin, ia_end);
+  int m0 = 0;
+  if ((rc = window_map_2d(ctx, a, pb.alg, s, W, &m0)) != MQP_OK) return rc;
   if (huge) {
     cudaError_t e = ctx->huge.ensure(mqp::piv2d_huge_scratch_bytes(ctx->device, 2 * pb.SM[0] + 1, 2 * pb.SM[1] + 1));
     if (e != cudaSuccess) return cuda_fail(ctx, e, "scratch of the 2D kernel for search windows above 128");
@@ -335,7 +327,7 @@ int run_pass_3d(mqp_ctx* ctx, const Problem& pb, const mqp_params* p, const void
   a.ia_end = ia_end;
   a.threshold = p->threshold;
   a.mask_threshold = p->mask_threshold;
-  if (!direct && need_g2 && !dSN && !dplanes) {
+  if (!direct && mqp::piv3d_takes_map(a, pb.alg)) {
     // window-sum map; without memory for it the kernels read the integral volumes
     e = ctx->wmap.ensure(mqp::window_map3_bytes(a, pb.alg));
     if (e == cudaErrorMemoryAllocation) {
@@ -574,15 +566,15 @@ static int host_pipelined_2d(mqp_ctx* ctx, const Problem& pb, const mqp_params* 
       return cuda_fail(ctx, e, "pipeline order");
     int rc = integrals_2d(ctx, pb, ctx->img1.ptr, ctx->img2.ptr, dtype, s, x0, x1);
     if (rc != MQP_OK) return rc;
-    if ((rc = window_map_2d(ctx, pb, dSN != nullptr, false, s, x1, &m0)) != MQP_OK) return rc;
+    mqp::Piv2dArgs a = args_2d(ctx, pb, p, ctx->img1.ptr, ctx->img2.ptr, mask ? ctx->mask.ptr : nullptr,
+                               mask_skip ? ctx->mask_skip.ptr : nullptr, dtype, dVF, dSN, nullptr, nullptr, 0, pb.n_ia);
+    if ((rc = window_map_2d(ctx, a, pb.alg, s, x1, &m0)) != MQP_OK) return rc;
     int64_t c1 = done_cols;
     while (c1 < vf2 && (x1 == W || need(c1) <= x1)) ++c1;
     if (c1 > done_cols) {
-      rc = launch_2d(ctx, args_2d(ctx, pb, p, ctx->img1.ptr, ctx->img2.ptr, mask ? ctx->mask.ptr : nullptr,
-                                  mask_skip ? ctx->mask_skip.ptr : nullptr, dtype, dVF, dSN, nullptr, nullptr,
-                                  vf1 * done_cols, vf1 * c1),
-                     pb.alg, s);
-      if (rc != MQP_OK) return rc;
+      a.ia_begin = vf1 * done_cols;
+      a.ia_end = vf1 * c1;
+      if ((rc = launch_2d(ctx, a, pb.alg, s)) != MQP_OK) return rc;
       if ((e = cudaEventRecord(ctx->pipe_ev[PIPE_PIECES + k], s)) != cudaSuccess) return cuda_fail(ctx, e, "pipeline order");
       outs.push_back({k, (size_t)(vf1 * done_cols), (size_t)(vf1 * (c1 - done_cols))});
       done_cols = c1;

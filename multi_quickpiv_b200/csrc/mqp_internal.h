@@ -40,8 +40,8 @@ struct WindowMap {
 WindowMap window_map(int H, int W, int IS1, int IS2, int SM1, int SM2, int alg, bool SN, void* base);
 cudaError_t launch_window_map(const double* II2, const double* II1, int H, int W, int IS1, int IS2, int SM1, int SM2,
                               const WindowMap& m, int m0, int m1, cudaStream_t s);
-// passes whose kernel takes the map
-bool piv2d_takes_map(int IS1, int IS2, int SM1, int SM2, int alg, bool SN, bool pred);
+// passes whose kernel reads a map and that have the lags to pay for it
+bool piv2d_takes_map(const Piv2dArgs& a, int alg);
 
 // The same for a column-major H x W x D volume: out is (H+1) x (W+1) x (D+1),
 // first plane zero; scratch holds integral3d_scratch_bytes(H, W, D) bytes.
@@ -163,7 +163,9 @@ cudaError_t launch_piv3d(const Piv3dArgs& a, int alg, long long chunk, cudaStrea
 size_t piv3d_shared_bytes(const int IS[3], const int SM[3], long long H, long long W);
 void piv3d_bind_shared(Piv3dArgs& a, int layers, char* base);
 // Window-sum map of an NSQECC or ZNCC pass without SN (geometry and integral
-// volumes set in `a`): bytes, and the kernel, which binds a.ws / a.wz to `base`.
+// volumes set in `a`): whether the pass takes one, its bytes, and the kernel,
+// which binds a.ws / a.wz to `base`.
+bool piv3d_takes_map(const Piv3dArgs& a, int alg);
 size_t window_map3_bytes(const Piv3dArgs& a, int alg);
 cudaError_t launch_window_map3(Piv3dArgs& a, int alg, void* base, cudaStream_t s);
 

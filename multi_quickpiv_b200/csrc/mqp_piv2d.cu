@@ -8,6 +8,7 @@
 
 #include <string>
 
+#include "mqp_finish.cuh"
 #include "mqp_internal.h"
 #include "mqp_stage.cuh"
 
@@ -105,11 +106,35 @@ cudaError_t launch_piv2d_batch(const Piv2dBatch& b, cudaStream_t s, std::string&
   return cudaErrorInvalidValue;
 }
 
-bool piv2d_takes_map(int IS1, int IS2, int SM1, int SM2, int alg, bool SN, bool pred) {
-  if (direct2d_ok(IS1, IS2, SM1, SM2) || piv2d_local_sums(IS1, IS2, SM1, SM2, alg)) return false;
-  // SN: only the strip kernel reads the map then
-  if (SN) return alg == ALG_NSQECC && !pred && IS1 <= 32 && IS2 <= 32 && piv2d_fft_len(IS1 + 2 * SM1, IS2 + 2 * SM2) == 64;
-  return alg == ALG_NSQECC || alg == ALG_ZNCC;
+bool piv2d_takes_map(const Piv2dArgs& a, int alg) {
+  if (alg != ALG_NSQECC && alg != ALG_ZNCC) return false;
+  if (direct2d_ok(a.IS1, a.IS2, a.SM1, a.SM2) || piv2d_local_sums(a.IS1, a.IS2, a.SM1, a.SM2, alg)) return false;
+  const int N = piv2d_fft_len(a.IS1 + 2 * a.SM1, a.IS2 + 2 * a.SM2);
+  if (N && piv2d_team_ok(N, a.IS1 <= N / 2 && a.IS2 <= N / 2, alg)) return false;
+  // with SN every lag is formed in full, and only the strip kernel reads a map
+  // for that; with planes none does
+  if (a.planes || (a.SN && !piv2d_strip_ok(a, alg))) return false;
+  // The map costs a pass over all window positions and saves each lag reads of
+  // the integral images.  It pays from some number of lags per position.  Whole
+  // passes at 2048^2 without and with it, us, next to the line:
+  //   NSQECC, length 32 (IS 16, SM 8): 1.1 lags 213, 227; 2.0 lags 345, 337
+  //           length 64 (IS 32, SM 16): 0.7 lags 164, 172; 1.1 lags 223, 221; 1.4 lags 245, 229
+  //           length 128 (IS 64, SM 32): 1.8 lags 489, 511; 2.5 lags 689, 679
+  //           length 256 (IS 128, SM 64): 1.0 lags 639, 711; 3.8 lags 1643, 1620
+  //           with SN (IS 32, SM 16): 1.06 lags 227, 228; 1.4 lags 334, 236
+  //   ZNCC, which saves twice the reads: length 64 (IS 24, SM 16) 0.26 lags 210, 226; 0.48 lags 261, 270;
+  //           0.67 lags 317, 310; length 128 0.26 lags 278, 292; 0.44 lags 365, 359; length 256 1.0 lags 661, 653
+  // And on a small image, whatever the number of areas, where one area's walk
+  // saves more time than the map takes: a thread's lags beyond the first few
+  // hide no latency, some 65,000 positions' worth each.  NSQECC IS 32, SM 16, step 48:
+  // 512^2 79, 74; 1024^2 83, 80; 1440^2 90.5, 91.1; SM 10, step 32: 512^2 58.5, 56.8; 768^2 59.0, 60.9;
+  // IS 16, SM 8, step 16: 256^2 47.4, 49.8; 512^2 47.4, 49.9; IS 64, SM 32, step 96: 640^2 90, 84; 1024^2 111, 109;
+  // 1440^2 119, 122; ZNCC IS 24, SM 16, step 48: 1024^2 119, 117; 1440^2 155, 169.
+  const double least = alg == ALG_ZNCC ? 0.5 : (N == 64 ? 1.0 : 2.0);
+  const double area_lags = (double)(2 * a.SM1 + 1) * (2 * a.SM2 + 1);
+  const double thread_lags = area_lags / (N == 32 || N == 64 ? 32 : (N == 128 ? 128 : 256));
+  const double positions = (double)winmap_ld(a.H, a.IS1, a.SM1) * winmap_ld(a.W, a.IS2, a.SM2);
+  return positions <= 65536.0 * (thread_lags - 9.0) || area_lags * (double)(a.ia_end - a.ia_begin) >= least * positions;
 }
 
 cudaError_t launch_piv2d(const Piv2dArgs& a, int alg, cudaStream_t s, std::string& err) {

@@ -787,6 +787,23 @@ __global__ void __launch_bounds__(256) window_map3_kernel(Piv3dArgs a, float2* w
 }
 }  // namespace
 
+bool piv3d_takes_map(const Piv3dArgs& a, int alg) {
+  if ((alg != ALG_NSQECC && alg != ALG_ZNCC) || !finish3_fast(a, alg)) return false;
+  const int n1 = winmap_ld(a.H, a.IS[0], a.SM[0]), n2 = winmap_ld(a.W, a.IS[1], a.SM[1]),
+            n3 = winmap_ld(a.D, a.IS[2], a.SM[2]);
+  if (n2 > 65535 || (n3 + ZMAP - 1) / ZMAP > 65535) return false;  // the map kernel's grid
+  // As in 2D (piv2d_takes_map); without a map the pass ends in the full K3c.
+  // Whole passes at 256x256x192 without and with it, us:
+  //   NSQECC, length 32 (IS 16, SM 8): 0.15 lags a position 337, 406; 0.37 lags 556, 562; 1.2 lags 1220, 929
+  //           length 64 (IS 32, SM 16): 1.1 lags 1228, 1410; 2.0 lags 1790, 1828; 7 lags 5575, 4569
+  //   ZNCC,   length 32: 0.15 lags 624, 710; 0.37 lags 821, 826; 1.2 lags 1503, 1189
+  //           length 64: 0.28 lags 974, 1069; 1.1 lags 1699, 1493
+  const int SS[3] = {a.IS[0] + 2 * a.SM[0], a.IS[1] + 2 * a.SM[1], a.IS[2] + 2 * a.SM[2]};
+  const double least = alg == ALG_NSQECC && piv3d_fft_len(SS) > 32 ? 2.5 : 0.4;
+  const double lags = (double)(a.ia_end - a.ia_begin) * (2 * a.SM[0] + 1) * (2 * a.SM[1] + 1) * (2 * a.SM[2] + 1);
+  return lags >= least * n1 * n2 * n3;
+}
+
 size_t window_map3_bytes(const Piv3dArgs& a, int alg) {
   const size_t n = (size_t)winmap_ld(a.H, a.IS[0], a.SM[0]) * (size_t)winmap_ld(a.W, a.IS[1], a.SM[1]) *
                    (size_t)winmap_ld(a.D, a.IS[2], a.SM[2]);
@@ -797,7 +814,6 @@ cudaError_t launch_window_map3(Piv3dArgs& a, int alg, void* base, cudaStream_t s
   a.ldw1 = winmap_ld(a.H, a.IS[0], a.SM[0]);
   a.ldw2 = winmap_ld(a.W, a.IS[1], a.SM[1]);
   const int n3 = winmap_ld(a.D, a.IS[2], a.SM[2]);
-  if (a.ldw2 > 65535 || (n3 + ZMAP - 1) / ZMAP > 65535) return cudaSuccess;  // no map: the integral volumes are read
   float2* ws = alg == ALG_ZNCC ? nullptr : (float2*)base;
   double2* wz = alg == ALG_ZNCC ? (double2*)base : nullptr;
   const int th = std::min(256, (a.ldw1 + 31) / 32 * 32);
