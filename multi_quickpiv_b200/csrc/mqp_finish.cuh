@@ -7,8 +7,8 @@
 // second-largest value, and evaluates in full (finish_one: the values every
 // other path forms) only what the approximation leaves open: one lag where
 // the largest approximate value is alone within PEAK_GAP of the maximum, the
-// whole box otherwise.  The result is the full search's: the approximations
-// are within 1.5e-6 of the values they stand for (below), so a lag more than
+// few there are or the whole box otherwise (settle_peak).  The result is the full search's: the approximations
+// are within 1.6e-6 of the values they stand for (below), so a lag more than
 // PEAK_GAP below the largest cannot be the maximum.
 //
 // NSQECC, v = d / (d + n) with d = sqrt(S2) sqrt(F2) and n = F2 + S2 - 2c
@@ -30,7 +30,7 @@
 
 namespace mqp {
 
-constexpr float PEAK_GAP = 1e-5f;
+constexpr float PEAK_GAP = 4e-6f;
 
 // ---------------------------------------------------------------------------
 // window-sum maps
@@ -111,7 +111,7 @@ MQP_HD MQP_FI float nsqecc_walk(float S2, float root, float c, float m2, float F
   return d * rcp_approx(den);
 }
 // Masked NSQECC, c1 = (F*mask)*G and S2 = mask*G^2; most keeps the largest
-// magnitude, above 8 = open.
+// magnitude, above 4 = open.
 MQP_HD MQP_FI float masked_walk(double S2, double c1, double sumF2, float sqF, float& most) {
   const float d = sqrt_approx(fabsf((float)S2)) * sqF;
   const double n = ((sumF2 - 2.0 * c1) + S2) + (double)d;
@@ -138,6 +138,129 @@ __device__ __forceinline__ void unmapped_lags(const LagRanges& R, int e1, int e2
   }
 }
 
+__device__ __forceinline__ float warp_most(float v) {
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, off));
+  return v;
+}
+
+// The largest value of NT threads (barriers around red when NT > 32).
+template <int NT>
+__device__ __forceinline__ float block_most(int tid, float v, double* red) {
+  v = warp_most(v);
+  if (NT > 32) {
+    float* rf = reinterpret_cast<float*>(red);
+    if ((tid & 31) == 0) rf[tid >> 5] = v;
+    __syncthreads();
+    v = rf[0];
+    for (int w = 1; w < NT / 32; ++w) v = fmaxf(v, rf[w]);
+    __syncthreads();
+  }
+  return v;
+}
+
+// FFTCC, whose values are exact: the first of equal maxima above 0.
+template <int NT>
+__device__ __forceinline__ int first_of(int tid, const TopTwo& t, double* red) {
+  const float mx = block_most<NT>(tid, t.b1, red);
+  if (!(mx > 0.f)) return -1;
+  int idx = t.b1 == mx ? t.idx : 0x7fffffff;
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) idx = min(idx, __shfl_xor_sync(0xffffffffu, idx, off));
+  if (NT > 32) {
+    int* ri = reinterpret_cast<int*>(red);
+    if ((tid & 31) == 0) ri[tid >> 5] = idx;
+    __syncthreads();
+    idx = ri[0];
+    for (int w = 1; w < NT / 32; ++w) idx = min(idx, ri[w]);
+    __syncthreads();
+  }
+  return idx;
+}
+
+// The peak from every thread's share t of the walk.  One lag alone within the
+// gap of the largest is the peak.  Of several, each thread evaluates its own in
+// full (sim); where a thread holds two, so that one's lag is not known, or
+// full is set, all lags of the box are.  Nearly equal maxima are ordinary where
+// an area holds noise on a bright background, and areas that take longer than
+// their neighbours also cost the persistent kernels' warps their common pace
+// through the code.  1024^2 passes, noise 100 wide on a background of 1000, whole
+// box for any two in a gap of 1e-5 -> this with PEAK_GAP: NSQECC IS 16, SM 8 292 -> 204 us
+// (every lag in full, no walk: 237), IS 12, SM 19 791 -> 415 (755), IS 32, SM 16 510 -> 408
+// (571), masked IS 32 2506 -> 1661 (1632).
+template <int NT, typename SIM>
+__device__ __forceinline__ int settle_peak(const LagRanges& R, int tid, int P1, bool full, const TopTwo& t, double* red,
+                                           SIM sim) {
+  const unsigned FULL = 0xffffffffu;
+  constexpr int NW = NT / 32;
+  const int warp = tid >> 5, lane = tid & 31;
+  float th = 0.f;
+  if (!full) {
+    const float mx = block_most<NT>(tid, t.b1, red);
+    if (!(mx > 0.f)) return -1;
+    th = mx * (1.f - PEAK_GAP);
+    // threads with a value within the gap, above the 16th bit those with two, and the lag of an only one
+    int cnt = (t.b1 >= th) + ((t.b2 >= th) << 16), idx = t.b1 >= th ? t.idx : -1;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      cnt += __shfl_xor_sync(FULL, cnt, off);
+      idx = max(idx, __shfl_xor_sync(FULL, idx, off));
+    }
+    if (NT > 32) {
+      int* ri = reinterpret_cast<int*>(red);
+      if (lane == 0) {
+        ri[2 * warp] = cnt;
+        ri[2 * warp + 1] = idx;
+      }
+      __syncthreads();
+      cnt = ri[0];
+      idx = ri[1];
+      for (int w = 1; w < NW; ++w) {
+        cnt += ri[2 * w];
+        idx = max(idx, ri[2 * w + 1]);
+      }
+      __syncthreads();
+    }
+    if (cnt == 1) return idx;
+    full = cnt >> 16;
+  }
+  double best = 0.0;
+  int bidx = -1;
+  // this thread's lags: its one, or every NT-th of the box row by row
+  const int w2 = R.hi2 - R.lo2 + 1, d1 = NT / w2, d2 = NT - d1 * w2;
+  const int left = full ? ((R.hi1 - R.lo1 + 1) * w2 - tid + NT - 1) / NT : (t.b1 >= th);
+  const int first = full ? tid / w2 : t.idx / P1, rest = full ? tid - first * w2 : t.idx - first * P1;
+  int s1 = full ? R.lo1 + first : rest, s2 = full ? R.lo2 + rest : first;
+#pragma unroll 1
+  for (int k = 0; k < left; ++k) {
+    peak_take(sim(s1, s2), s1 + P1 * s2, best, bidx);
+    s1 += d1;
+    s2 += d2;
+    if (s2 > R.hi2) {
+      s2 -= w2;
+      ++s1;
+    }
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    const double ob = __shfl_xor_sync(FULL, best, off);
+    const int oi = __shfl_xor_sync(FULL, bidx, off);
+    peak_merge(best, bidx, ob, oi);
+  }
+  if (NT > 32) {
+    if (lane == 0) {
+      red[2 * warp] = best;
+      red[2 * warp + 1] = (double)bidx;
+    }
+    __syncthreads();
+    best = red[0];
+    bidx = (int)red[1];
+    for (int w = 1; w < NW; ++w) peak_merge(best, bidx, red[2 * w], (int)red[2 * w + 1]);
+    __syncthreads();
+  }
+  return bidx;
+}
+
 // Lag box walk of NT threads (one warp, or a block whose every thread calls
 // it).  cc(s1, s2) * scale is the raw correlation.  Returns the first maximum > 0
 // in column-major order (bidx = s1 + P1 s2, -1 = none) on every thread.  Window
@@ -149,7 +272,6 @@ template <int ALG, int NT, int LWN, typename CC>
 __device__ __forceinline__ int finish_search(const Piv2dArgs& a, const IAGeom& g, const IAScalars& sc,
                                              const LagRanges& R, int tid, int P1, double scale, CC cc,
                                              const double* lw, double* red) {
-  const unsigned FULL = 0xffffffffu;
   static_assert(ALG == ALG_FFTCC || ALG == ALG_ZNCC || ALG == ALG_NSQECC, "unmasked similarities");
   const float sqF = sqrtf((float)sc.sumF2), F2 = (float)sc.sumF2;
   const float fscale = (float)scale, m2 = -2.f * fscale;
@@ -298,102 +420,22 @@ __device__ __forceinline__ int finish_search(const Piv2dArgs& a, const IAGeom& g
     }
   }
   if (open < 0) top_open(t);
-  // the largest value of the box, and what comes within the gap of it
-  float* redf = reinterpret_cast<float*>(red);
-  const int warp = tid >> 5, lane = tid & 31;
-  constexpr int NW = NT / 32;
-  float mx = t.b1;
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(FULL, mx, off));
-  if (NT > 32) {
-    if (lane == 0) redf[warp] = mx;
-    __syncthreads();
-    mx = redf[0];
-    for (int w = 1; w < NW; ++w) mx = fmaxf(mx, redf[w]);
-    __syncthreads();
-  }
-  if (!full) {
-    if (!(mx > 0.f)) return -1;
-    if (ALG == ALG_FFTCC) {  // exact values: the first of equal maxima
-      int idx = t.b1 == mx ? t.idx : 0x7fffffff;
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) idx = min(idx, __shfl_xor_sync(FULL, idx, off));
-      if (NT > 32) {
-        int* ri = reinterpret_cast<int*>(red);
-        if (lane == 0) ri[warp] = idx;
-        __syncthreads();
-        idx = ri[0];
-        for (int w = 1; w < NW; ++w) idx = min(idx, ri[w]);
-        __syncthreads();
-      }
-      return idx;
-    }
-    const float th = mx * (1.f - PEAK_GAP);
-    // how many threads hold a value within the gap (one that holds two counts
-    // as two), and the lag of the only one
-    int cnt = (t.b1 >= th) + (t.b2 >= th), idx = t.b1 >= th ? t.idx : -1;
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      cnt += __shfl_xor_sync(FULL, cnt, off);
-      idx = max(idx, __shfl_xor_sync(FULL, idx, off));
-    }
-    if (NT > 32) {
-      int* ri = reinterpret_cast<int*>(red);
-      if (lane == 0) {
-        ri[2 * warp] = cnt;
-        ri[2 * warp + 1] = idx;
-      }
-      __syncthreads();
-      cnt = ri[0];
-      idx = ri[1];
-      for (int w = 1; w < NW; ++w) {
-        cnt += ri[2 * w];
-        idx = max(idx, ri[2 * w + 1]);
-      }
-      __syncthreads();
-    }
-    if (cnt == 1) return idx;
-  }
-  double best = 0.0;
-  int bidx = -1;
-  const int w2 = R.hi2 - R.lo2 + 1, all = (R.hi1 - R.lo1 + 1) * w2;
-#pragma unroll 1
-  for (int q = tid; q < all; q += NT) {
-    const int s1 = R.lo1 + q / w2, s2 = R.lo2 + q % w2;
-    peak_take(finish_one<ALG, LWN>(a, g, sc, s1, s2, (double)cc(s1, s2) * scale, 0.0, lw), s1 + P1 * s2, best, bidx);
-  }
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    const double ob = __shfl_xor_sync(FULL, best, off);
-    const int oi = __shfl_xor_sync(FULL, bidx, off);
-    peak_merge(best, bidx, ob, oi);
-  }
-  if (NT > 32) {
-    if (lane == 0) {
-      red[2 * warp] = best;
-      red[2 * warp + 1] = (double)bidx;
-    }
-    __syncthreads();
-    best = red[0];
-    bidx = (int)red[1];
-    for (int w = 1; w < NW; ++w) peak_merge(best, bidx, red[2 * w], (int)red[2 * w + 1]);
-    __syncthreads();
-  }
-  return bidx;
+  if (ALG == ALG_FFTCC) return first_of<NT>(tid, t, red);
+  return settle_peak<NT>(R, tid, P1, full, t, red, [&](int s1, int s2) {
+    return finish_one<ALG, LWN>(a, g, sc, s1, s2, (double)cc(s1, s2) * scale, 0.0, lw);
+  });
 }
 
 // finish_search of masked NSQECC (masked_nsqecc_ops.jl:123-142): c1(s1, s2) is
 // (F*mask)*G and c2 is mask*G^2, the window sum.  Both carry the FP32 transforms'
 // error, so the denominator may cancel where the mask covers little: it is
-// formed in FP64 as in similarity_value, and a value above 8 of either sign (a
+// formed in FP64 as in similarity_value, and a value above 4 of either sign (a
 // cancelled denominator, which scales the square root's approximation up and
-// may come out of it with the other sign) takes the full search.
+// may come out of it with the other sign) takes the full search: up to there
+// the root's 3e-7 leaves the value within 1.2e-6, its other steps add 4e-7.
 template <int NT, typename C1, typename C2>
 __device__ __forceinline__ int finish_search_masked(const Piv2dArgs& a, const IAGeom& g, const IAScalars& sc,
                                                     const LagRanges& R, int tid, int P1, C1 c1, C2 c2, double* red) {
-  const unsigned FULL = 0xffffffffu;
-  constexpr int NW = NT / 32;
-  const int warp = tid >> 5, lane = tid & 31;
   if (sc.sumF2 == 0.0) return -1;  // no lag has a value above 0
   const float sqF = sqrtf((float)sc.sumF2);
   const bool full = !(sc.sumF2 > 1e-30 && sc.sumF2 < 1e30);
@@ -416,72 +458,10 @@ __device__ __forceinline__ int finish_search_masked(const Piv2dArgs& a, const IA
       }
     }
   }
-  if (most > 8.f) top_open(t);
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    const float o1 = __shfl_xor_sync(FULL, t.b1, off), o2 = __shfl_xor_sync(FULL, t.b2, off);
-    const int oi = __shfl_xor_sync(FULL, t.idx, off);
-    if (o1 > t.b1) {
-      t.b2 = fmaxf(t.b1, o2);
-      t.b1 = o1;
-      t.idx = oi;
-    } else {
-      // of equal ones every lane keeps the same: they end in the full search
-      if (o1 == t.b1) t.idx = max(t.idx, oi);
-      t.b2 = fmaxf(t.b2, o1);
-    }
-  }
-  if (NT > 32) {
-    float* rf = reinterpret_cast<float*>(red);
-    if (lane == 0) {
-      rf[3 * warp] = t.b1;
-      rf[3 * warp + 1] = t.b2;
-      rf[3 * warp + 2] = __int_as_float(t.idx);
-    }
-    __syncthreads();
-    t.b1 = t.b2 = 0.f;
-    t.idx = -1;
-    for (int w = 0; w < NW; ++w) {
-      const float o1 = rf[3 * w], o2 = rf[3 * w + 1];
-      if (o1 > t.b1) {
-        t.b2 = fmaxf(t.b1, o2);
-        t.b1 = o1;
-        t.idx = __float_as_int(rf[3 * w + 2]);
-      } else {
-        t.b2 = fmaxf(t.b2, o1);
-      }
-    }
-    __syncthreads();
-  }
-  if (!full) {
-    if (!(t.b1 > 0.f)) return -1;
-    if (t.b2 < t.b1 * (1.f - PEAK_GAP)) return t.idx;
-  }
-  double best = 0.0;
-  int bidx = -1;
-#pragma unroll 1
-  for (int q = tid; q < total; q += NT) {
-    const int s1 = R.lo1 + q / w2, s2 = R.lo2 + q % w2;
-    peak_take(finish_one<ALG_MASK_NSQECC>(a, g, sc, s1, s2, c2(s1, s2), c1(s1, s2)), s1 + P1 * s2, best, bidx);
-  }
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    const double ob = __shfl_xor_sync(FULL, best, off);
-    const int oi = __shfl_xor_sync(FULL, bidx, off);
-    peak_merge(best, bidx, ob, oi);
-  }
-  if (NT > 32) {
-    if (lane == 0) {
-      red[2 * warp] = best;
-      red[2 * warp + 1] = (double)bidx;
-    }
-    __syncthreads();
-    best = red[0];
-    bidx = (int)red[1];
-    for (int w = 1; w < NW; ++w) peak_merge(best, bidx, red[2 * w], (int)red[2 * w + 1]);
-    __syncthreads();
-  }
-  return bidx;
+  if (most > 4.f) top_open(t);
+  return settle_peak<NT>(R, tid, P1, full, t, red, [&](int s1, int s2) {
+    return finish_one<ALG_MASK_NSQECC>(a, g, sc, s1, s2, c2(s1, s2), c1(s1, s2));
+  });
 }
 
 // Whether a pass ends in finish_search (masked: finish_search_masked).

@@ -116,21 +116,22 @@ bool piv2d_takes_map(const Piv2dArgs& a, int alg) {
   if (a.planes || (a.SN && !piv2d_strip_ok(a, alg))) return false;
   // The map costs a pass over all window positions and saves each lag reads of
   // the integral images.  It pays from some number of lags per position.  Whole
-  // passes at 2048^2 without and with it, us, next to the line:
-  //   NSQECC, length 32 (IS 16, SM 8): 1.1 lags 213, 227; 2.0 lags 345, 337
-  //           length 64 (IS 32, SM 16): 0.7 lags 164, 172; 1.1 lags 223, 221; 1.4 lags 245, 229
-  //           length 128 (IS 64, SM 32): 1.8 lags 489, 511; 2.5 lags 689, 679
-  //           length 256 (IS 128, SM 64): 1.0 lags 639, 711; 3.8 lags 1643, 1620
-  //           with SN (IS 32, SM 16): 1.06 lags 227, 228; 1.4 lags 334, 236
-  //   ZNCC, which saves twice the reads: length 64 (IS 24, SM 16) 0.26 lags 210, 226; 0.48 lags 261, 270;
-  //           0.67 lags 317, 310; length 128 0.26 lags 278, 292; 0.44 lags 365, 359; length 256 1.0 lags 661, 653
+  // passes at 2048^2 (an image against itself moved, plus noise) without and with it, us,
+  // next to the line:
+  //   NSQECC, length 32 (IS 16, SM 8): 0.5 lags 153, 157; 0.7 lags 177, 177; 1.1 lags 239, 223
+  //           length 64 (IS 32, SM 16): 0.27 lags 126, 136; 0.48 lags 167, 169; 0.67 lags 207, 201
+  //           length 128 (IS 64, SM 32): 0.26 lags 195, 203; 0.44 lags 267, 263; 1.0 lags 400, 378
+  //           length 256 (IS 128, SM 64): 1.0 lags 578, 552; 3.8 lags 1682, 1623
+  //           with SN (IS 32, SM 16): 1.06 lags 258, 246; 1.4 lags 358, 259
+  //   ZNCC,   length 64 (IS 24, SM 16): 0.26 lags 232, 249; 0.48 lags 285, 292; 0.67 lags 340, 334
+  //           length 128: 0.26 lags 296, 312; 0.44 lags 379, 379; 1.0 lags 522, 503
   // And on a small image, whatever the number of areas, where one area's walk
   // saves more time than the map takes: a thread's lags beyond the first few
   // hide no latency, some 65,000 positions' worth each.  NSQECC IS 32, SM 16, step 48:
-  // 512^2 79, 74; 1024^2 83, 80; 1440^2 90.5, 91.1; SM 10, step 32: 512^2 58.5, 56.8; 768^2 59.0, 60.9;
-  // IS 16, SM 8, step 16: 256^2 47.4, 49.8; 512^2 47.4, 49.9; IS 64, SM 32, step 96: 640^2 90, 84; 1024^2 111, 109;
-  // 1440^2 119, 122; ZNCC IS 24, SM 16, step 48: 1024^2 119, 117; 1440^2 155, 169.
-  const double least = alg == ALG_ZNCC ? 0.5 : (N == 64 ? 1.0 : 2.0);
+  // 512^2 71, 63; 1024^2 77, 73; 1440^2 91.5, 89.6; SM 10, step 32: 512^2 58.6, 59.3 (58.5, 56.8 in another
+  // run); 768^2 67.7, 66.6 (59.0, 60.9); IS 16, SM 8, step 16: 256^2 56.7, 59.4; 640^2 56.7, 59.6; IS 64, SM 32,
+  // step 96: 640^2 97, 91; 1024^2 103, 99; 1440^2 125, 146; ZNCC IS 24, SM 16, step 48: 768^2 115, 113; 1440^2 173, 183.
+  const double least = a.SN ? 1.0 : (N == 32 ? 0.8 : 0.5);
   const double area_lags = (double)(2 * a.SM1 + 1) * (2 * a.SM2 + 1);
   const double thread_lags = area_lags / (N == 32 || N == 64 ? 32 : (N == 128 ? 128 : 256));
   const double positions = (double)winmap_ld(a.H, a.IS1, a.SM1) * winmap_ld(a.W, a.IS2, a.SM2);

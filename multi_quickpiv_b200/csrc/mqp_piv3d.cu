@@ -337,6 +337,38 @@ __global__ void k3c_merge_kernel(Piv3dArgs a, long long n, int parts) {
   k3c_final(a, g, ci, lag_ranges3(a, g), b, bi, mx, sum);
 }
 
+// Last lags whose sums the pass's map holds.
+__device__ __forceinline__ void mapped_lags3(const Piv3dArgs& a, const IAGeom3& g, const LagRanges3& R, int (&e)[3]) {
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const int size = d == 0 ? a.H : (d == 1 ? a.W : a.D);
+    e[d] = min(R.hi[d], lag_mapped_max(a.SM[d], a.IS[d], g.g0[d], g.hi[d], size));
+  }
+}
+
+// The walk's value of one lag (k3c_walk_kernel's) from its raw correlation; a
+// lag that the map does not hold: +inf.
+template <int ALG>
+__device__ __forceinline__ float walk_value3(const Piv3dArgs& a, const IAGeom3& g, const IA3State& st, const int (&e)[3],
+                                             int s1, int s2, int s3, float sqF, float fscale, float c) {
+  if (s1 > e[0] || s2 > e[1] || s3 > e[2]) return INFINITY;
+  const long long w = (g.g0[0] + s1 + a.SM[0]) +
+                      (long long)a.ldw1 * ((g.g0[1] + s2 + a.SM[1]) + (long long)a.ldw2 * (g.g0[2] + s3 + a.SM[2]));
+  if (ALG == ALG_NSQECC) {
+    const float2 m = __ldg(a.ws + w);
+    int open = 0;
+    return nsqecc_walk(m.x, m.y, c, -2.f * fscale, (float)st.sumF2, sqF, open);
+  }
+  int r0, r1, c0, c1, z0, z1;
+  lag_window(s1, a.IS[0], g.g0[0], g.lo[0], g.hi[0], r0, r1);
+  lag_window(s2, a.IS[1], g.g0[1], g.lo[1], g.hi[1], c0, c1);
+  lag_window(s3, a.IS[2], g.g0[2], g.lo[2], g.hi[2], z0, z1);
+  const double n = (double)(r1 - r0) * (double)(c1 - c0) * (double)(z1 - z0);
+  const double2 m = __ldg(a.wz + w);
+  const double SG = m.x - 2.0 * st.meanG * m.y + n * st.meanG * st.meanG;
+  return c * fscale * rsqrtf((float)(SG > 0.0 ? SG : 0.0));
+}
+
 // K3c of a pass that ends in the walk (finish3_fast): the lag pair's inverse
 // along k3, the raw correlations to V (the fit's neighbourhood), FP32
 // approximations of the similarity to the block's two largest.  With the
@@ -356,13 +388,8 @@ __global__ void __launch_bounds__(K3C_THREADS, N <= 64 ? 2 : 1) k3c_walk_kernel(
   const LagRanges3 R = lag_ranges3(a, g);
   const float sqF = sqrtf((float)st.sumF2), F2 = (float)st.sumF2;
   const float fscale = (float)cc_scale3<N>(), m2 = -2.f * fscale;
-  const bool map = ALG == ALG_NSQECC ? a.ws != nullptr : (ALG == ALG_ZNCC && a.wz != nullptr);
-  int e[3];  // last lags whose sums the map holds (without a map: none)
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    const int size = d == 0 ? a.H : (d == 1 ? a.W : a.D);
-    e[d] = map ? min(R.hi[d], lag_mapped_max(a.SM[d], a.IS[d], g.g0[d], g.hi[d], size)) : R.lo[d] - 1;
-  }
+  int e[3];
+  mapped_lags3(a, g, R, e);
   TopTwo t;
   t.b1 = t.b2 = 0.f;
   t.idx = -1;
@@ -460,11 +487,11 @@ __global__ void __launch_bounds__(K3C_THREADS, N <= 64 ? 2 : 1) k3c_walk_kernel(
 
 // A block per IA: the walk's parts, every lag in full where they leave more
 // than one open, and the Gaussian fit with a lane per neighbour.
-constexpr int K3F_THREADS = 128;
+constexpr int K3F_THREADS = 512;  // at most
 template <int N, int ALG>
 __global__ void __launch_bounds__(K3F_THREADS) k3c_walk_merge_kernel(Piv3dArgs a, int parts) {
   const long long ci = blockIdx.x, ia = a.ia_begin + ci;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, NT = blockDim.x, lane = tid & 31, warp = tid >> 5;
   const IA3State st = a.state[ci];
   if (st.skip) {
     if (tid == 0) k3c_skipped(a, ci);
@@ -493,10 +520,47 @@ __global__ void __launch_bounds__(K3F_THREADS) k3c_walk_merge_kernel(Piv3dArgs a
     bidx = -1;
     const int n1 = R.hi[0] - R.lo[0] + 1, n2 = R.hi[1] - R.lo[1] + 1, n3 = R.hi[2] - R.lo[2] + 1;
     const int total = n1 > 0 && n2 > 0 && n3 > 0 ? n1 * n2 * n3 : 0;
-    for (int q = tid; q < total; q += K3F_THREADS) {
-      const int s1 = R.lo[0] + q % n1, s2 = R.lo[1] + (q / n1) % n2, s3 = R.lo[2] + q / (n1 * n2);
-      const int idx = s1 + P1 * s2 + P12 * s3;
-      peak_take(full_sim3<ALG>(a, g, st, s1, s2, s3, (double)V[idx] * scale), idx, best, bidx);
+    // Within the bounds of the approximations only the lags that they put in the
+    // gap are evaluated: the box is walked again, a batch of values in flight.
+    // Nearly equal maxima are ordinary where an area holds noise on a bright
+    // background, and one block with the whole box in full (33^3 lags of 64
+    // bytes) held its pass up: 128^3 NSQECC, IS 32, SM 16, step 16, noise 1056 -> 738 us.
+    const bool every = !(st.sumF2 > 1e-30 && st.sumF2 < 1e30) || !(t.b1 < INFINITY);
+    const float th = t.b1 * (1.f - PEAK_GAP), sqF = sqrtf((float)st.sumF2);
+    int e[3];
+    mapped_lags3(a, g, R, e);
+    // lag (s1, s2, s3) of this thread, every NT-th of the box
+    const int d1 = NT % n1, d2 = (NT / n1) % n2, d3 = NT / (n1 * n2);
+    int s1 = R.lo[0] + tid % n1, s2 = R.lo[1] + (tid / n1) % n2, s3 = R.lo[2] + tid / (n1 * n2);
+    auto step = [&]() {
+      s1 += d1;
+      s2 += d2;
+      s3 += d3;
+      if (s1 > R.hi[0]) {
+        s1 -= n1;
+        ++s2;
+      }
+      if (s2 > R.hi[1]) {
+        s2 -= n2;
+        ++s3;
+      }
+    };
+    constexpr int B = 4;
+#pragma unroll 1
+    for (int q0 = tid; q0 < total; q0 += B * NT) {
+      int lag[B];  // those to evaluate, -1 = not
+#pragma unroll
+      for (int k = 0; k < B; ++k) {
+        lag[k] = s3 <= R.hi[2] ? s1 + P1 * s2 + P12 * s3 : -1;
+        if (!every && lag[k] >= 0 && !(walk_value3<ALG>(a, g, st, e, s1, s2, s3, sqF, (float)scale, V[lag[k]]) >= th)) lag[k] = -1;
+        step();
+      }
+#pragma unroll
+      for (int k = 0; k < B; ++k) {
+        if (lag[k] < 0) continue;
+        const int u3 = lag[k] / P12, u2 = (lag[k] - u3 * P12) / P1, u1 = lag[k] - u3 * P12 - u2 * P1;
+        peak_take(full_sim3<ALG>(a, g, st, u1, u2, u3, (double)V[lag[k]] * scale), lag[k], best, bidx);
+      }
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
@@ -513,7 +577,7 @@ __global__ void __launch_bounds__(K3F_THREADS) k3c_walk_merge_kernel(Piv3dArgs a
     __syncthreads();
     best = rb[0];
     bidx = ri[0];
-    for (int w = 1; w < K3F_THREADS / 32; ++w) peak_merge(best, bidx, rb[w], ri[w]);
+    for (int w = 1; w < NT / 32; ++w) peak_merge(best, bidx, rb[w], ri[w]);
   }
   if (warp != 0) return;
   double r[3] = {-1.0, -1.0, -1.0};  // no peak: 1-based (0, 0, 0), displacement -(SM+1)
@@ -620,7 +684,10 @@ cudaError_t run_chunks(Piv3dArgs a, long long chunk, cudaStream_t s, std::string
       if (finish3_fast(a, ALG) && (ALG == ALG_FFTCC || (ALG == ALG_ZNCC ? a.wz != nullptr : a.ws != nullptr))) {
         const int th = walk_threads((P12 + cparts - 1) / cparts);
         k3c_walk_kernel<N, ALG><<<dim3(cparts, (unsigned)n), th, 0, s>>>(a);
-        k3c_walk_merge_kernel<N, ALG><<<(unsigned)n, K3F_THREADS, 0, s>>>(a, cparts);
+        // few areas: more threads each, for the boxes walked again (96^3 of 125 areas, all near ties: 597 us with
+        // 128 threads, 471 with 512); many: 160^3, two passes, 2530 us with 128, 2570 with 512
+        const int ft = ALG != ALG_FFTCC && n <= 1024 ? K3F_THREADS : 128;
+        k3c_walk_merge_kernel<N, ALG><<<(unsigned)n, ft, 0, s>>>(a, cparts);
         done = true;
       }
     }
@@ -794,12 +861,12 @@ bool piv3d_takes_map(const Piv3dArgs& a, int alg) {
   if (n2 > 65535 || (n3 + ZMAP - 1) / ZMAP > 65535) return false;  // the map kernel's grid
   // As in 2D (piv2d_takes_map); without a map the pass ends in the full K3c.
   // Whole passes at 256x256x192 without and with it, us:
-  //   NSQECC, length 32 (IS 16, SM 8): 0.15 lags a position 337, 406; 0.37 lags 556, 562; 1.2 lags 1220, 929
-  //           length 64 (IS 32, SM 16): 1.1 lags 1228, 1410; 2.0 lags 1790, 1828; 7 lags 5575, 4569
-  //   ZNCC,   length 32: 0.15 lags 624, 710; 0.37 lags 821, 826; 1.2 lags 1503, 1189
-  //           length 64: 0.28 lags 974, 1069; 1.1 lags 1699, 1493
+  //   NSQECC, length 32 (IS 16, SM 8): 0.15 lags a position 392, 431; 0.37 lags 612, 571; 1.2 lags 1276, 939
+  //           length 64 (IS 32, SM 16): 0.28 lags 655, 755; 1.1 lags 1282, 1101 (160^3 468, 511); 2.0 lags 1837, 1484
+  //   ZNCC,   length 32: 0.15 lags 677, 770; 0.37 lags 875, 892; 1.2 lags 1555, 1242
+  //           length 64: 0.28 lags 1034, 1123; 1.1 lags 1748, 1546 (160^3 702, 745); 2.0 lags 2972, 2378
   const int SS[3] = {a.IS[0] + 2 * a.SM[0], a.IS[1] + 2 * a.SM[1], a.IS[2] + 2 * a.SM[2]};
-  const double least = alg == ALG_NSQECC && piv3d_fft_len(SS) > 32 ? 2.5 : 0.4;
+  const double least = piv3d_fft_len(SS) > 32 ? 1.2 : 0.4;
   const double lags = (double)(a.ia_end - a.ia_begin) * (2 * a.SM[0] + 1) * (2 * a.SM[1] + 1) * (2 * a.SM[2] + 1);
   return lags >= least * n1 * n2 * n3;
 }

@@ -20,12 +20,12 @@ def _scans(ctx, call):
 
 # FFT lengths 32, 64 (strips, one warp per area), 128 and 256 on both sides of their lines (lags a position; small
 # images); with SN strips alone read one (steps up to the window, at most 36 lag rows)
-CASES_2D = [(512, "nsqecc", 16, 8, 10, False, True), (512, "nsqecc", 16, 8, 16, False, False),
-            (1536, "nsqecc", 32, 16, 24, False, True), (1536, "nsqecc", 32, 16, 40, False, False),
+CASES_2D = [(512, "nsqecc", 16, 8, 10, False, True), (512, "nsqecc", 16, 8, 24, False, False),
+            (1536, "nsqecc", 32, 16, 24, False, True), (1536, "nsqecc", 32, 16, 64, False, False),
             (512, "nsqecc", 32, 16, 40, False, True), (640, "nsqecc", 32, 10, 32, False, False),
-            (1536, "nsqecc", 64, 32, 32, False, True), (1536, "nsqecc", 64, 32, 64, False, False),
+            (1536, "nsqecc", 64, 32, 32, False, True), (1536, "nsqecc", 64, 32, 128, False, False),
             (512, "nsqecc", 64, 32, 64, False, True),
-            (1800, "nsqecc", 100, 60, 60, False, True), (1800, "nsqecc", 100, 60, 100, False, False),
+            (1800, "nsqecc", 100, 60, 60, False, True), (1800, "nsqecc", 100, 60, 250, False, False),
             (512, "nsqecc", 32, 16, 8, True, True), (512, "nsqecc", 32, 16, 33, True, False),
             (512, "nsqecc", 12, 19, 12, True, False), (512, "nsqecc", 64, 32, 32, True, False),
             (1536, "zncc", 24, 16, 32, False, True), (1536, "zncc", 24, 16, 64, False, False),
@@ -49,7 +49,7 @@ def test_planes_take_none(gpu):
 
 @pytest.mark.parametrize("alg,IS,SM,st,sn,formed", [
     ("nsqecc", 16, 8, 8, False, True), ("nsqecc", 16, 8, 40, False, False), ("nsqecc", 16, 8, 8, True, False),
-    ("nsqecc", 24, 16, 12, False, True), ("nsqecc", 24, 16, 24, False, False),
+    ("nsqecc", 24, 16, 12, False, True), ("nsqecc", 24, 16, 36, False, False),
     ("zncc", 16, 8, 8, False, True), ("zncc", 16, 8, 40, False, False), ("fft", 16, 8, 8, False, False)])
 def test_3d(alg, IS, SM, st, sn, formed, gpu):
     import torch

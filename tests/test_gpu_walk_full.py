@@ -52,3 +52,28 @@ def test_bright_pixels_beside_dark_windows(shape, IS, SM, st, seed, gpu):
     b[tuple(g.integers(0, np.array(shape), (int(np.prod(shape)) // (1500 if nd == 2 else 20000), nd)).T)] = 1e9
     _walk_equals_full(a.astype(np.float32), b.astype(np.float32), corr_alg="nsqecc", interSize=(IS,) * nd,
                       searchMargin=(SM,) * nd, step=(st,) * nd)
+
+
+# FFT lengths 32, 64 (strips, one warp per area), 128 and 256 in 2D; 32, 64 and 128 in 3D
+@pytest.mark.parametrize("shape,IS,SM,st", [((437, 391), 16, 8, 6), ((437, 391), 32, 16, 9), ((437, 391), 24, 12, 25),
+                                            ((437, 391), 64, 30, 21), ((437, 391), 100, 60, 50),
+                                            ((101, 93, 85), 16, 8, 8), ((101, 93, 85), 32, 16, 15),
+                                            ((101, 93, 85), 40, 25, 20)])
+@pytest.mark.parametrize("alg", ["nsqecc", "zncc", "mask"])
+@pytest.mark.parametrize("kind", ["noise", "period", "flat"])
+def test_near_ties(shape, IS, SM, st, alg, kind, gpu):
+    """Noise on a bright background, whose similarities lie within a few
+    rounding steps of one another, several equal maxima, and every lag equal."""
+    nd, g = len(shape), np.random.default_rng(11)
+    if alg == "mask" and IS == 100:
+        pytest.skip("no masks above 128")
+    if kind == "noise":
+        i1, i2 = 3000 + 20 * g.uniform(size=shape), 3000 + 20 * g.uniform(size=shape)
+    elif kind == "period":
+        i1 = np.tile(g.uniform(0, 9, (8,) * nd), [s // 8 + 1 for s in shape])[tuple(slice(0, s) for s in shape)]
+        i2 = i1
+    else:
+        i1 = i2 = np.full(shape, 7.0)
+    mask = (g.uniform(size=shape) < 0.7).astype(np.float32) if alg == "mask" else None
+    _walk_equals_full(i1.astype(np.float32), i2.astype(np.float32), mask, corr_alg="nsqecc" if alg == "mask" else alg,
+                      interSize=(IS,) * nd, searchMargin=(SM,) * nd, step=(st,) * nd)

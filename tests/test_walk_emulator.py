@@ -60,7 +60,7 @@ def test_masked_approximation(emu, F2):
     g = np.random.default_rng(4)
     S2 = F2 * 10 ** g.uniform(-6, 6, 4000) * np.where(g.uniform(size=4000) < 0.1, -1, 1)  # the transforms' error has no sign
     d = np.sqrt(np.abs(S2) * F2)
-    share = g.uniform(0.15, 3, 4000) * np.where(g.uniform(size=4000) < 0.3, -1, 1)  # denominator / d
+    share = g.uniform(0.3, 3, 4000) * np.where(g.uniform(size=4000) < 0.3, -1, 1)  # denominator / d
     c1 = (F2 + S2 + d - share * d) / 2
     emu.mqp_walk_masked.restype = C.c_float
 
@@ -69,9 +69,9 @@ def test_masked_approximation(emu, F2):
         return emu.mqp_walk_masked(4000, _p(S2), _p(c1), C.c_double(F2), _p(walk), _p(full)), walk, full
 
     most, walk, full = run(c1)
-    assert most <= 8
+    assert most <= 4
     assert np.max(np.abs(walk / full - 1)) < 4 * EPS32  # the same denominator; reciprocal and product against a quotient
     for part in (0.1, 1e-3, 1e-6, -1e-6, -1e-3, -0.1):
         cb, at = c1.copy(), g.integers(0, 4000)
         cb[at] = (F2 + S2[at] + d[at] - part * d[at]) / 2
-        assert run(cb)[0] > 8
+        assert run(cb)[0] > 4
