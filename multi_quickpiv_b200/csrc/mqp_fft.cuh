@@ -86,6 +86,17 @@ MQP_HD MQP_FI float2 cmulc(float2 a, float2 b) {
 }
 MQP_HD MQP_FI float2 cscale(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
 
+// A column that carries two real rows' spectra as A + iB: conj(F) G of both, as
+// PA + i PB, at a bin from that bin's values and its mirror's (unconjugated).
+// packed_mirror: the mirror of bin 2m + h of 2M among the bins of parity h.
+MQP_HD MQP_FI int packed_mirror(int M, int h, int m) { return h ? M - 1 - m : (M - m) & (M - 1); }
+MQP_HD MQP_FI float2 packed_product(float2 G, float2 Gm, float2 F, float2 Fm) {
+  const float2 Gn = cconj(Gm), Fn = cconj(Fm);
+  const float2 A = cscale(cadd(G, Gn), 0.5f), B = cscale(cmul_mi(csub(G, Gn)), 0.5f);
+  const float2 Af = cscale(cadd(F, Fn), 0.5f), Bf = cscale(cmul_mi(csub(F, Fn)), 0.5f);
+  return cadd(cmulc(Af, A), cmul_pi(cmulc(Bf, B)));
+}
+
 // a * exp(sign * 2*pi*i * m / L), sign = -1 forward, +1 inverse.  Multiples
 // of a quarter or an eighth turn take their exact short forms.
 template <int L, bool INV>

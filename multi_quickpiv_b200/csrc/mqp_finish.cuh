@@ -52,6 +52,25 @@ MQP_HD MQP_FI int lag_mapped_max(int SM, int IS, int g0, int hi, int size) {
   return last < 2 * SM ? last : 2 * SM;
 }
 
+// The lags of the box that the map does not hold: the rows past e1, then what
+// the others have past column e2.
+struct UnmappedLags {
+  int w2, rows, h1, cols;  // lags of a row, lags in rows past e1, rows up to e1, lags past column e2
+  MQP_HD MQP_FI int count() const { return rows + cols; }
+  MQP_HD MQP_FI void at(const LagRanges& R, int q, int& s1, int& s2) const {
+    s1 = q < rows ? R.hi1 - q / w2 : R.lo1 + (q - rows) % h1;
+    s2 = q < rows ? R.lo2 + q % w2 : R.hi2 - (q - rows) / h1;
+  }
+};
+MQP_HD MQP_FI UnmappedLags unmapped_lags(const LagRanges& R, int e1, int e2) {
+  UnmappedLags u;
+  u.w2 = R.hi2 - R.lo2 + 1;
+  u.rows = R.hi1 > e1 ? (R.hi1 - (e1 > R.lo1 - 1 ? e1 : R.lo1 - 1)) * u.w2 : 0;
+  u.h1 = e1 - R.lo1 + 1;
+  u.cols = R.hi2 > e2 && u.h1 > 0 ? (R.hi2 - (e2 > R.lo2 - 1 ? e2 : R.lo2 - 1)) * u.h1 : 0;
+  return u;
+}
+
 // a lane's two largest values and the lag index of the largest
 struct TopTwo {
   float b1, b2;
@@ -124,19 +143,6 @@ MQP_HD MQP_FI float masked_walk(double S2, double c1, double sumF2, float sqF, f
 MQP_HD MQP_FI void top_open(TopTwo& t) { t.b1 = t.b2 = INFINITY; }
 
 #if defined(__CUDACC__)
-
-// The lags of the box that the map does not hold (rows past e1, then columns
-// past e2), over the lanes.
-template <typename F>
-__device__ __forceinline__ void unmapped_lags(const LagRanges& R, int e1, int e2, int lane, F take) {
-  const int w2 = R.hi2 - R.lo2 + 1, nr = R.hi1 > e1 ? (R.hi1 - (e1 > R.lo1 - 1 ? e1 : R.lo1 - 1)) * w2 : 0;
-  const int h1 = e1 - R.lo1 + 1, nc = R.hi2 > e2 && h1 > 0 ? (R.hi2 - (e2 > R.lo2 - 1 ? e2 : R.lo2 - 1)) * h1 : 0;
-#pragma unroll 1
-  for (int q = lane; q < nr + nc; q += 32) {
-    if (q < nr) take(R.hi1 - q / w2, R.lo2 + q % w2);
-    else take(R.lo1 + (q - nr) % h1, R.hi2 - (q - nr) / h1);
-  }
-}
 
 __device__ __forceinline__ float warp_most(float v) {
 #pragma unroll
@@ -408,13 +414,11 @@ __device__ __forceinline__ int finish_search(const Piv2dArgs& a, const IAGeom& g
     }
   }
   if (!full && map) {
-    // the lags the map does not hold: rows past e1, then columns past e2
-    const int w2 = R.hi2 - R.lo2 + 1, nr = R.hi1 > e1 ? (R.hi1 - max(e1, R.lo1 - 1)) * w2 : 0;
-    const int h1 = e1 - R.lo1 + 1, nc = R.hi2 > e2 && h1 > 0 ? (R.hi2 - max(e2, R.lo2 - 1)) * h1 : 0;
+    const UnmappedLags u = unmapped_lags(R, e1, e2);
 #pragma unroll 1
-    for (int q = tid; q < nr + nc; q += NT) {
-      const int s1 = q < nr ? R.hi1 - q / w2 : R.lo1 + (q - nr) % h1;
-      const int s2 = q < nr ? R.lo2 + q % w2 : R.hi2 - (q - nr) / h1;
+    for (int q = tid; q < u.count(); q += NT) {
+      int s1, s2;
+      u.at(R, q, s1, s2);
       const float v = (float)finish_one<ALG>(a, g, sc, s1, s2, (double)cc(s1, s2) * scale);
       top_take(t, ALG == ALG_ZNCC ? v * sqF : v, s1 + P1 * s2);  // on the walk's scale
     }

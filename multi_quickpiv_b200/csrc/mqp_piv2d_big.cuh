@@ -234,12 +234,8 @@ MQP_HD MQP_FI void big_col_product(int t, const float2* S, const float2* SF, flo
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
       const int m = (t & 31) + 32 * k;
-      const int mm = h ? MB - 1 - m : (MB - m) & (MB - 1);
-      const float2 Zk = G0[m], Zn = cconj(G0[mm]);
-      const float2 Fk = F[m], Fn = cconj(F[mm]);
-      const float2 A = cscale(cadd(Zk, Zn), 0.5f), B = cscale(cmul_mi(csub(Zk, Zn)), 0.5f);
-      const float2 Af = cscale(cadd(Fk, Fn), 0.5f), Bf = cscale(cmul_mi(csub(Fk, Fn)), 0.5f);
-      q[k] = cadd(cmulc(Af, A), cmul_pi(cmulc(Bf, B)));
+      const int mm = packed_mirror(MB, h, m);
+      q[k] = packed_product(G0[m], G0[mm], F[m], F[mm]);
     }
     __syncwarp();
     PK[MB * h + (t & 31)] = q[0];
@@ -262,12 +258,8 @@ MQP_HD MQP_FI void big_col_product(int t, const float2* S, const float2* SF, flo
     for (int m = 0; m < MB; ++m) F[m] = f[fpos<MB>(m)];
 #pragma unroll 4
     for (int m = 0; m < MB; ++m) {
-      const int mm = h ? MB - 1 - m : (MB - m) & (MB - 1);
-      const float2 Zk = G[m], Zn = cconj(G[mm]);
-      const float2 Fk = F[m], Fn = cconj(F[mm]);
-      const float2 A = cscale(cadd(Zk, Zn), 0.5f), B = cscale(cmul_mi(csub(Zk, Zn)), 0.5f);
-      const float2 Af = cscale(cadd(Fk, Fn), 0.5f), Bf = cscale(cmul_mi(csub(Fk, Fn)), 0.5f);
-      p[m] = cadd(cmulc(Af, A), cmul_pi(cmulc(Bf, B)));
+      const int mm = packed_mirror(MB, h, m);
+      p[m] = packed_product(G[m], G[mm], F[m], F[mm]);
     }
   }
 #endif

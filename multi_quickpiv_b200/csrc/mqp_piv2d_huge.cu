@@ -106,30 +106,17 @@ __device__ __forceinline__ void huge_ia(const Piv2dArgs& a, long long ia, float2
   }
 
   // ---- B: columns, a thread quad per column (quarter q warp-uniform) ----
-  // A round's G and F columns come into shared memory as coalesced tiles: read
-  // from the scratch slot by the columns' own threads, 32 lanes touched 32
-  // lines per load and the quad of a column read each of them four times
-  // (3,721 IAs of window 256: 7045 -> 5478 us with the lag rows' tile below).
   float2* ft = sm + HugeSmem::FT;
   for (int r = 0; r < 2; ++r) {
-    const int col = t % 64, q = t / 64, k2 = 64 * r + col;
-    const float2* gsrc = GS + (long long)(64 * r) * NH;
-    const float2* fsrc = FS + (long long)(64 * r) * MH;
-#pragma unroll 16
-    for (int c = 0; c < 64; ++c) park[c * HugeSmem::TG + t] = gsrc[c * NH + t];
-#pragma unroll 16
-    for (int c = t / MH; c < 64; c += 2) ft[c * HugeSmem::TF + t % MH] = fsrc[c * MH + t % MH];
+    huge_b_tiles(r, t, GS, FS, park, ft);
     __syncthreads();
-    float2* mine = park + q * 64 + col;
     float2 f[QH];
     {
       float2 y[QH];
-      huge_col_g(q, park + col * HugeSmem::TG, tw, y);
+      huge_b_g(t, park, tw, y);
       __syncthreads();  // the tile is read: the park slots take its place
-      huge_col_park(y, mine);
+      huge_b_f(r, t, y, ft, tw, park, pack, f);
     }
-    huge_col_f(q, ft + col * HugeSmem::TF, tw, f);
-    if (k2 == 0) huge_col_pack(q, mine, f, pack);
     __syncthreads();
     huge_b_part2(r, t, tw, park, pack, f);
     __syncthreads();
@@ -142,10 +129,9 @@ __device__ __forceinline__ void huge_ia(const Piv2dArgs& a, long long ia, float2
   {
     const float scale = (float)cc_scale<NH>();
     const int hh = t / MH;
-    const bool tiled = P1 * HugeSmem::LS <= HugeSmem::PARK;
+    const bool tiled = huge_c_tiled(P1);
     if (tiled) {
-#pragma unroll 8
-      for (int s1 = t / MH; s1 < P1; s1 += 2) park[s1 * HugeSmem::LS + t % MH] = LG[(long long)s1 * MH + t % MH];
+      huge_c_tile(t, P1, LG, park);
       __syncthreads();
     }
     for (int b = 0; b < P1; b += MH) {

@@ -275,12 +275,7 @@ MQP_HD MQP_FI void huge_col_product(int k2, int q, float2* park, const float2* p
   const float2* Fp = pack + NH;
   for (int m = 0; m < QH; ++m) {
     const int k = 4 * m + q, kn = (NH - k) & (NH - 1);
-    const float2 Zk = Gp[k], Zn = cconj(Gp[kn]);
-    const float2 Fk = Fp[k], Fn = cconj(Fp[kn]);
-    const float2 A = cscale(cadd(Zk, Zn), 0.5f), B = cscale(cmul_mi(csub(Zk, Zn)), 0.5f);
-    const float2 Af = cscale(cadd(Fk, Fn), 0.5f), Bf = cscale(cmul_mi(csub(Fk, Fn)), 0.5f);
-    const float2 PA = cmulc(Af, A), PB = cmulc(Bf, B);
-    park[m * HPS] = cconj(cadd(PA, cmul_pi(PB)));
+    park[m * HPS] = cconj(packed_product(Gp[k], Gp[kn], Fp[k], Fp[kn]));
   }
 }
 
@@ -322,10 +317,37 @@ MQP_HD MQP_FI void huge_col_combine(int k2, int p, int P1, const float2* xch, fl
 }
 
 // Stage B for thread t in round r (columns k2 = 64 r + t % 64, quarter
-// q = t / 64): part 1, then (block barrier) part 2, then (block barrier)
-// part 3, then a block barrier before the next round reuses the park.
-// park: 64 columns x 4 quarters x 64 values (HugeSmem); the quad of column c
-// exchanges through its own slots, based at park[c].
+// q = t / 64): the tiles, G, F, part 2, part 3, with a block barrier after each
+// and before the next round reuses the park.  park: first the G tile, then 64
+// columns x 4 quarters x 64 values (HugeSmem); the quad of column c exchanges
+// through its own slots, based at park[c].  ft: the F tile.
+//
+// A round's G and F columns come into shared memory as coalesced tiles: read
+// from the scratch slot by the columns' own threads, 32 lanes touched 32
+// lines per load and the quad of a column read each of them four times
+// (3,721 IAs of window 256: 7045 -> 5478 us with the lag rows' tile).
+MQP_HD MQP_FI void huge_b_tiles(int r, int t, const float2* GS, const float2* FS, float2* park, float2* ft) {
+  const float2* gsrc = GS + (long long)(64 * r) * NH;
+  const float2* fsrc = FS + (long long)(64 * r) * MH;
+#pragma unroll 16
+  for (int c = 0; c < 64; ++c) park[c * HugeSmem::TG + t] = gsrc[c * NH + t];
+#pragma unroll 16
+  for (int c = t / MH; c < 64; c += 2) ft[c * HugeSmem::TF + t % MH] = fsrc[c * MH + t % MH];
+}
+MQP_HD MQP_FI void huge_b_g(int t, const float2* park, const float2* tw, float2 (&y)[QH]) {
+  huge_col_g(t / 64, park + t % 64 * HugeSmem::TG, tw, y);
+}
+// y takes the G tile's place
+MQP_HD MQP_FI void huge_b_f(int r, int t, const float2 (&y)[QH], const float2* ft, const float2* tw, float2* park,
+                            float2* pack, float2 (&f)[QH]) {
+  const int col = t % 64, q = t / 64;
+  float2* mine = park + q * 64 + col;
+  huge_col_park(y, mine);
+  huge_col_f(q, ft + col * HugeSmem::TF, tw, f);
+  if (64 * r + col == 0) huge_col_pack(q, mine, f, pack);
+}
+// The tiles, G and F in one for host code whose threads run one after another
+// (a tile under another thread's slots would be lost): columns from the slot.
 MQP_HD MQP_FI void huge_b_part1(int r, int t, const float2* GS, const float2* FS, const float2* tw, float2* park,
                                 float2* pack, float2 (&f)[QH]) {
   const int col = t % 64, q = t / 64, k2 = r * 64 + col;
@@ -351,7 +373,13 @@ MQP_HD MQP_FI void huge_b_part3(int r, int t, int P1, const float2* park, float2
 // ---------------------------------------------------------------------------
 // stage C: lag row s1, half hh of the complex-to-real inverse along k2
 // ---------------------------------------------------------------------------
-// As team_phase3_row with the row's spectrum X[u] = LG[s1 * ls + u].
+// As team_phase3_row with the row's spectrum X[u] = LG[s1 * ls + u].  Thread t's
+// share of the rows' tile (stride HugeSmem::LS), for up to 191 lag rows:
+MQP_HD MQP_FI bool huge_c_tiled(int P1) { return P1 * HugeSmem::LS <= HugeSmem::PARK; }
+MQP_HD MQP_FI void huge_c_tile(int t, int P1, const float2* LG, float2* park) {
+#pragma unroll 8
+  for (int s1 = t / MH; s1 < P1; s1 += 2) park[s1 * HugeSmem::LS + t % MH] = LG[(long long)s1 * MH + t % MH];
+}
 MQP_HD MQP_FI void huge_lag_row(int s1, int hh, int P1, int P2, const float2* LG, float* cc, float scale, int ls = MH) {
   mqp_no_hoist();
   constexpr int M = MH, Q = QH;

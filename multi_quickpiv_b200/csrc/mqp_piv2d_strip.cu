@@ -232,12 +232,8 @@ __device__ __forceinline__ void strip_product(int lane, int h, uint32_t tm, floa
   }
   __syncwarp();
   {
-    const int mm = h ? M - 1 - lane : (M - lane) & (M - 1);  // the mirror bin, in the same half
-    const float2 Zk = pk[lane], Zn = cconj(pk[mm]), Fk = pk[M + lane], Fn = cconj(pk[M + mm]);
-    const float2 A = cscale(cadd(Zk, Zn), 0.5f), B = cscale(cmul_mi(csub(Zk, Zn)), 0.5f);
-    const float2 Af = cscale(cadd(Fk, Fn), 0.5f), Bf = cscale(cmul_mi(csub(Fk, Fn)), 0.5f);
-    const float2 PA = cmulc(Af, A), PB = cmulc(Bf, B);
-    pk[2 * M + lane] = cconj(cadd(PA, cmul_pi(PB)));
+    const int mm = packed_mirror(M, h, lane);
+    pk[2 * M + lane] = cconj(packed_product(pk[lane], pk[mm], pk[M + lane], pk[M + mm]));
   }
   __syncwarp();
 #pragma unroll
@@ -326,9 +322,13 @@ __device__ __noinline__ void strip_finish(const Piv2dArgs& a, int v1, int v2, do
           const long long w = w0 + s1 + (long long)a.ldw * s2;
           take(s1, s2, sim(__ldg(&a.ws[w].y), __ldg(a.wd + w), cc(s1, s2)));
         }
-      unmapped_lags(R, e1, e2, lane, [&](int s1, int s2) {
+      const UnmappedLags u = unmapped_lags(R, e1, e2);
+#pragma unroll 1
+      for (int q = lane; q < u.count(); q += 32) {
+        int s1, s2;
+        u.at(R, q, s1, s2);
         take(s1, s2, (float)finish_one<ALG>(a, g, sc, s1, s2, (double)cc(s1, s2) * scale));
-      });
+      }
     } else {
       const int w2 = R.hi2 - R.lo2 + 1, total = (R.hi1 - R.lo1 + 1) * w2;
 #pragma unroll 1
