@@ -32,6 +32,8 @@ int mqp_create(mqp_ctx** out, int device) {
   if (e != cudaSuccess) return fail(nullptr, MQP_ERR_CUDA, std::string("cudaSetDevice: ") + cudaGetErrorString(e));
   mqp_ctx* c = new mqp_ctx();
   c->device = device;
+  for (DevBuf* b : c->buffers())
+    if (b != &c->wmap) b->spare = &c->wmap;  // passes run without a map
   e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) {
     delete c;
@@ -45,11 +47,7 @@ int mqp_destroy(mqp_ctx* ctx) {
   if (!ctx) return MQP_OK;
   cudaSetDevice(ctx->device);
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-  for (DevBuf* b : {&ctx->img1, &ctx->img2, &ctx->mask, &ctx->mask_skip, &ctx->II1, &ctx->IIg, &ctx->IIg2, &ctx->wmap,
-                    &ctx->VF, &ctx->SN, &ctx->pred, &ctx->planes, &ctx->status, &ctx->iscratch,
-                    &ctx->scratch3d, &ctx->passVF[0], &ctx->passVF[1], &ctx->post_in, &ctx->post_mask,
-                    &ctx->post_out, &ctx->post_outf, &ctx->post_mask_out, &ctx->post_scratch})
-    b->release();
+  for (DevBuf* b : ctx->buffers()) b->release();
   for (cudaStream_t st : {ctx->in_stream, ctx->out_stream})
     if (st) {
       cudaStreamSynchronize(st);
@@ -209,11 +207,13 @@ int run_pass_2d(mqp_ctx* ctx, const Problem& pb, const mqp_params* p, const void
   int rc = integrals_2d(ctx, pb, d1, d2, dtype, s, 0, W);
   if (rc != MQP_OK) return rc;
   mqp::Piv2dArgs a = args_2d(ctx, pb, p, d1, d2, dmask, dskip, dtype, dVF, dSN, dpred, dplanes, ia_begin, ia_end);
+  cudaError_t e;
+  if (huge && (e = ctx->huge.ensure(mqp::piv2d_huge_scratch_bytes(ctx->device, 2 * pb.SM[0] + 1, 2 * pb.SM[1] + 1))) != cudaSuccess)
+    return cuda_fail(ctx, e, "scratch of the 2D kernel for search windows above 128");
+  // the map last: a buffer grown after it might take its memory
   int m0 = 0;
   if ((rc = window_map_2d(ctx, a, pb.alg, s, W, &m0)) != MQP_OK) return rc;
   if (huge) {
-    cudaError_t e = ctx->huge.ensure(mqp::piv2d_huge_scratch_bytes(ctx->device, 2 * pb.SM[0] + 1, 2 * pb.SM[1] + 1));
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "scratch of the 2D kernel for search windows above 128");
     a.huge = (float2*)ctx->huge.ptr;
     std::string err;
     {

@@ -22,12 +22,18 @@ inline thread_local std::string g_create_error;
 struct DevBuf {
   void* ptr = nullptr;
   size_t bytes = 0;
+  DevBuf* spare = nullptr;  // given up when there is no memory for this buffer
   cudaError_t ensure(size_t n) {
     if (n <= bytes) return cudaSuccess;
     if (ptr) cudaFree(ptr);
     ptr = nullptr;
     bytes = 0;
     cudaError_t e = cudaMalloc(&ptr, n);
+    if (e == cudaErrorMemoryAllocation && spare && spare->ptr) {
+      cudaGetLastError();
+      spare->release();  // cudaFree waits for the kernels that read it
+      e = cudaMalloc(&ptr, n);
+    }
     if (e == cudaSuccess) bytes = n;
     return e;
   }
@@ -51,6 +57,11 @@ struct mqp_ctx {
   mqp_host::DevBuf huge;        // scratch slots of the 2D kernel for search windows above 128
   mqp_host::DevBuf post_in, post_mask, post_out, post_outf, post_mask_out, post_scratch;
   mqp_host::DevBuf traj_in, traj_out;  // host-array pseudo-trajectories
+  std::vector<mqp_host::DevBuf*> buffers() {
+    return {&img1, &img2, &mask, &mask_skip, &II1, &IIg, &IIg2, &wmap, &VF, &SN, &pred, &planes, &status, &iscratch,
+            &scratch3d, &passVF[0], &passVF[1], &def1, &def2, &huge, &post_in, &post_mask, &post_out, &post_outf,
+            &post_mask_out, &post_scratch, &traj_in, &traj_out};
+  }
   // host-array 2D path: copy-in and copy-out streams, events of its pieces
   cudaStream_t in_stream = nullptr, out_stream = nullptr;
   std::vector<cudaEvent_t> pipe_ev;
