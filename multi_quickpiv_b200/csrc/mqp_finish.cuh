@@ -320,6 +320,8 @@ __device__ __forceinline__ int finish_search(const Piv2dArgs& a, const IAGeom& g
         constexpr int B = 8;
         if (NT == 32 && w1 > 20) {
           // most of a warp's lanes find a row of their own: no index to keep per lag
+          // (2048^2 NSQECC strips, step 8, rows and lags dealt out: 33 rows 1277, 1299 us; 17 rows
+          // 1146, 1134; between them within 2 % of one another either way)
           const int s1 = min(R.lo1 + tid, e1);
           const bool mine = R.lo1 + tid <= e1;
 #pragma unroll 1

@@ -313,8 +313,9 @@ MQP_HD MQP_FI void row_process(const Piv2dArgs& a, const IAScalars& sc, int PASS
     if (PASS == PASS_PLAIN) {
       // loaded FB at a time before any is used, at addresses clamped into the
       // row: one by one under their conditions they cost a round trip each
-      // (1501x1999 ZNCC 567 -> 529 us); whole rows do not fit beside the next
-      // row's prefetch (737), nor do the masked passes' three images (390 -> 482)
+      // (1501x1999 ZNCC 567 -> 529 us, in another run 552 -> 521); whole rows do
+      // not fit beside the next row's prefetch (737), nor do the masked passes'
+      // three images (390 -> 482)
       constexpr int FB = 16;
 #pragma unroll
       for (int b = 0; b < FLIM; b += FB) {

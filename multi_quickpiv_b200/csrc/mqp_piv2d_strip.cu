@@ -16,14 +16,16 @@
 // memory (tcgen05.st / tcgen05.ld, 128 columns per block), which leaves the
 // registers to one transform at a time.  The lag spectra and the correlation
 // plane take the rows' place in shared memory once the block is through with
-// them, so a block needs 41 KB (step 8) to 78 KB (step 32) and twelve warps
-// fit on an SM, where the other kernel's 26 KB per warp and 255 registers fit
-// eight.  Each value goes through the same operations in the same order as
-// there: the fields are the same bit for bit.
+// them, so a block needs 42 KB at step 8 and three blocks, twelve warps, fit on
+// an SM, where the other kernel's 26 KB per warp and 255 registers fit eight
+// warps.  (A block takes up to 81 KB; past 75 KB - interSize 32, margin 16, from
+// step 29 - two blocks fit.)  Each correlation and similarity goes through the
+// same operations in the same order as there, so the vectors are the same bit
+// for bit; SN's FP64 sum over the lags runs in another order.
 //
-// Bound by instruction issue and supply (ncu, 1024^2 NSQECC step 8): 11.6k warp
+// Bound by instruction issue and supply (ncu, 1024^2 NSQECC step 8): 11.7k warp
 // instructions per IA (15.3k before), issue active 54 %, stalls led by
-// no_instruction (0.95 warps per issue) and wait (0.93).  Measured on B200 (kernel,
+// wait (0.93 warps per issue) and no_instruction (0.91).  Measured on B200 (kernel,
 // one warp per IA -> strips): 2048^2 NSQECC step 8 2113 -> 1202 us, FFTCC 1270 ->
 // 1023; 1024x1280 NSQECC step 16 199 -> 93; 2048^2 NSQECC step 16 with SN 589 ->
 // 354; 256^2 FFTCC Float64 step 16 35 -> 17.
@@ -49,7 +51,6 @@ constexpr int SM_ = SN_ / 2;       // spectrum columns per IA: one per lane
 // block of eight warps and IAs (all before the rows loaded in batches); block
 // sizes that are not a multiple of four warps load the SM's quarters unevenly.
 constexpr int STRIP_WARPS = 4, STRIP_BLOCKS = 3;
-constexpr size_t STRIP_SMEM = 220 * 1024;  // of the 227 KB a block can have
 
 // Shared-memory layout of a block (float2 units unless said otherwise) and
 // the strip's shape.
@@ -668,14 +669,16 @@ cudaError_t launch_piv2d_strip(const Piv2dArgs& a, int alg, cudaStream_t s, std:
   int dev = 0;
   cudaGetDevice(&dev);
   const int sms = device_sm_count(dev);
-  // Strips of four fill the SMs from STRIP_BLOCKS blocks of four IAs each;
-  // a pass of no more IAs than blocks takes two warps to an IA instead.
-  // Measured (kernel): 225 IAs 20.9 us in strips of four, 18.6 as pairs of
-  // warps; 256 IAs (interSize 32, margin 10) 36 and 27 us (now 17 and 23).
+  // A pass whose IAs all run at once, one to a block, takes two warps to an IA:
+  // the kernel is one IA's latency then.  Past that the pairs start a second
+  // wave, strips of four do not.  Measured, strips of four and pairs: kernel, 225 IAs
+  // 20.9 and 18.6 us, 256 IAs (interSize 32, margin 10) 36 and 27 us (before the rows
+  // loaded in batches; now 17 and 23 as pairs); whole call, 484 IAs 63 and 73 us,
+  // 1024 IAs 64 and 95 (up to 441 IAs 63 either way: there the call's host work
+  // hides the kernel).  A block's shared memory is within bounds for all that
+  // piv2d_strip_ok lets through (80,896 bytes at most).
   const int wpi = n_ia <= (long long)STRIP_BLOCKS * sms ? 2 : 1;
-  int n = wpi == 2 ? 1 : 4;
-  StripCfg c = strip_cfg(a, n, wpi);
-  while (c.bytes > STRIP_SMEM && n > 1) c = strip_cfg(a, n = n / 2, wpi);
+  StripCfg c = strip_cfg(a, wpi == 2 ? 1 : 4, wpi);
   c.v2_0 = (int)(a.ia_begin / a.vf1);
   return alg == ALG_FFTCC ? strip_dt<ALG_FFTCC>(a, c, s, err) : strip_dt<ALG_NSQECC>(a, c, s, err);
 }

@@ -147,7 +147,9 @@ __global__ void __launch_bounds__(256) k3s_lines_kernel(Piv3dArgs a) {
   }
 }
 
-// With shared z-spectra: an IA's skip maximum and sumF2, a block per IA.
+// With shared z-spectra: an IA's skip maximum and sumF2, a block per IA.  The FP64
+// sum adds lines where k3a_kernel adds pixels over a thread's lines, so the two
+// sumF2 agree to FP64 rounding; the similarities' FP32 quotients rarely show it.
 template <typename T, int ALG>
 __global__ void __launch_bounds__(K3A_THREADS) k3s_state_kernel(Piv3dArgs a) {
   const long long ci = blockIdx.x;
