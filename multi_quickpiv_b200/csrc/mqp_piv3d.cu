@@ -862,14 +862,22 @@ bool piv3d_takes_map(const Piv3dArgs& a, int alg) {
             n3 = winmap_ld(a.D, a.IS[2], a.SM[2]);
   if (n2 > 65535 || (n3 + ZMAP - 1) / ZMAP > 65535) return false;  // the map kernel's grid
   // As in 2D (piv2d_takes_map); without a map the pass ends in the full K3c.
-  // Whole passes at 256x256x192 without and with it, us:
+  // Whole passes without and with it, us, at 256x256x192 unless said otherwise:
   //   NSQECC, length 32 (IS 16, SM 8): 0.15 lags a position 392, 431; 0.37 lags 612, 571; 1.2 lags 1276, 939
-  //           length 64 (IS 32, SM 16): 0.28 lags 655, 755; 1.1 lags 1282, 1101 (160^3 468, 511); 2.0 lags 1837, 1484
+  //           length 64 (IS 32, SM 16): 0.28 lags 655, 755; 1.1 lags 1282, 1101; 2.0 lags 1837, 1484
   //   ZNCC,   length 32: 0.15 lags 677, 770; 0.37 lags 875, 892; 1.2 lags 1555, 1242
-  //           length 64: 0.28 lags 1034, 1123; 1.1 lags 1748, 1546 (160^3 702, 745); 2.0 lags 2972, 2378
+  //           length 64: 0.28 lags 1034, 1123; 0.8 lags (IS 24, SM 12, 303x239x110) 1187, 1098; 1.1 lags 1748, 1546
+  // Up to length 64 it takes more areas than SMs as well: of fewer, the full K3c
+  // runs all at once.  NSQECC, length 64: 125 areas 1.1 lags (160^3) 468, 511; 4.9 lags
+  // (96^3) 371, 401; 216 areas 1.9 lags (160^3) 694, 605; length 32: 64 areas 1.1 lags (64^3) 92, 98;
+  // 216 areas 1.2 lags (96^3) 148, 139.  Length 128 (IS 48, SM 24), whose areas take
+  // several blocks: 27 areas 3.5 lags (96^3) 854, 783.
   const int SS[3] = {a.IS[0] + 2 * a.SM[0], a.IS[1] + 2 * a.SM[1], a.IS[2] + 2 * a.SM[2]};
-  const double least = piv3d_fft_len(SS) > 32 ? 1.2 : 0.4;
-  const double lags = (double)(a.ia_end - a.ia_begin) * (2 * a.SM[0] + 1) * (2 * a.SM[1] + 1) * (2 * a.SM[2] + 1);
+  const int N = piv3d_fft_len(SS);
+  const double least = N == 64 ? 0.6 : 0.4, areas = (double)(a.ia_end - a.ia_begin);
+  int dev = 0;
+  if (N <= 64 && cudaGetDevice(&dev) == cudaSuccess && areas <= device_sm_count(dev)) return false;
+  const double lags = areas * (2 * a.SM[0] + 1) * (2 * a.SM[1] + 1) * (2 * a.SM[2] + 1);
   return lags >= least * n1 * n2 * n3;
 }
 

@@ -49,7 +49,7 @@ def test_planes_take_none(gpu):
 
 @pytest.mark.parametrize("alg,IS,SM,st,sn,formed", [
     ("nsqecc", 16, 8, 8, False, True), ("nsqecc", 16, 8, 40, False, False), ("nsqecc", 16, 8, 8, True, False),
-    ("nsqecc", 24, 16, 12, False, True), ("nsqecc", 24, 16, 36, False, False),
+    ("nsqecc", 24, 16, 12, False, True), ("nsqecc", 24, 16, 36, False, False), ("nsqecc", 24, 16, 18, False, False),
     ("zncc", 16, 8, 8, False, True), ("zncc", 16, 8, 40, False, False), ("fft", 16, 8, 8, False, False)])
 def test_3d(alg, IS, SM, st, sn, formed, gpu):
     import torch
