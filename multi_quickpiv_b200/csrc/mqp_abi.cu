@@ -207,13 +207,12 @@ int run_pass_2d(mqp_ctx* ctx, const Problem& pb, const mqp_params* p, const void
   int rc = integrals_2d(ctx, pb, d1, d2, dtype, s, 0, W);
   if (rc != MQP_OK) return rc;
   mqp::Piv2dArgs a = args_2d(ctx, pb, p, d1, d2, dmask, dskip, dtype, dVF, dSN, dpred, dplanes, ia_begin, ia_end);
-  cudaError_t e;
-  if (huge && (e = ctx->huge.ensure(mqp::piv2d_huge_scratch_bytes(ctx->device, 2 * pb.SM[0] + 1, 2 * pb.SM[1] + 1))) != cudaSuccess)
-    return cuda_fail(ctx, e, "scratch of the 2D kernel for search windows above 128");
-  // the map last: a buffer grown after it might take its memory
   int m0 = 0;
   if ((rc = window_map_2d(ctx, a, pb.alg, s, W, &m0)) != MQP_OK) return rc;
   if (huge) {
+    cudaError_t e = ctx->huge.ensure(mqp::piv2d_huge_scratch_bytes(ctx->device, 2 * pb.SM[0] + 1, 2 * pb.SM[1] + 1));
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "scratch of the 2D kernel for search windows above 128");
+    if (!ctx->wmap.ptr) a.ws = nullptr, a.wd = nullptr, a.wz = nullptr;  // the map gave way
     a.huge = (float2*)ctx->huge.ptr;
     std::string err;
     {
